@@ -24,7 +24,7 @@ import ctypes as C
 import torch
 import torch.nn as nn
 
-from . import _cabi
+from . import _bqq_torch, _cabi
 from ._cabi import BqqLayer, check, lib
 
 _DTYPE_CODE = {torch.float32: _cabi.F32, torch.bfloat16: _cabi.BF16, torch.float16: _cabi.F16}
@@ -58,6 +58,8 @@ def _workspace(device: torch.device, kind: str, nbytes: int) -> torch.Tensor:
         size = max(int(nbytes), 256)
         buf = torch.zeros(size, dtype=torch.uint8, device=device)
         _WORKSPACES[key] = buf
+        if kind in ('decode', 'prefill'):          # the native forward finds it by device, stream and kind
+            _bqq_torch.set_scratch(key[0], key[1], int(kind == 'prefill'), buf.data_ptr(), buf.numel())
     return buf
 
 
@@ -99,6 +101,8 @@ def _require_cuda(t: torch.Tensor, what: str) -> None:
 class _BqqForwardMixin:
     """Shared engine of BinaryQuadratic and PackedBinaryQuadratic."""
 
+    _PLANE_SOURCES = None          # buffer names of _plane_sources() in an nn.Module; None: no native forward
+
     # -- packed state -------------------------------------------------------
     def _state(self) -> _PackedState:
         st = self.__dict__.get('_bqq_state')
@@ -110,6 +114,7 @@ class _BqqForwardMixin:
     def __getstate__(self):
         state = self.__dict__.copy()
         state.pop('_bqq_state', None)      # derived GPU state never enters a pickle
+        state.pop('_bqq_fast', None)
         return state
 
     def _dims(self):
@@ -141,7 +146,19 @@ class _BqqForwardMixin:
                 st.zsum = torch.empty(n * self.z_col, dtype=torch.uint8, device=device)
                 self._build_planes(st, device)
             st.plane_key = pkey
+            self._open_native(st)
         return st
+
+    def _open_native(self, st: _PackedState) -> None:
+        """Hand the packed state to the native forward (csrc/bqq_torch.cpp), which uses it for as long as the buffers
+        the planes were packed from are unchanged."""
+        if self._PLANE_SOURCES is None:
+            return
+        d = st.dims
+        n0, n1 = self._PLANE_SOURCES
+        t0, t1 = self._plane_sources()
+        self.__dict__['_bqq_fast'] = _bqq_torch.make_layer((d.bw, d.rw, d.cw, d.P, d.Q, d.r), st.zplanes, st.yplanes,
+                                                           n0, t0, n1, t1)
 
     def _layer(self, st: _PackedState) -> BqqLayer:
         """Descriptor handed to the C ABI; coefficient pointers are the live parameters."""
@@ -184,6 +201,9 @@ class _BqqForwardMixin:
                     'graph; call it under torch.no_grad() (training workflows need the reference module)')
 
     def forward(self, X):
+        Y = _bqq_torch.forward(self.__dict__, X)       # None: not the plain case (or an error to be raised below)
+        if Y is not None:
+            return Y
         self._check_inference_only(X)
         if X.dtype not in _DTYPE_CODE:
             # the reference computes in whatever float type X has (src/bqq_modules.py:35); the kernels
@@ -260,6 +280,9 @@ class _BqqForwardMixin:
 
         The prologue runs in fp32 on the unrounded values.  Up to 16 rows this is one decode call; larger
         batches apply the same operations with torch ops and call forward()."""
+        Y = _bqq_torch.forward_fused(self.__dict__, X, rms_weight, eps, swiglu, residual)
+        if Y is not None:
+            return Y
         self._check_inference_only(X)
         if rms_weight is not None and swiglu:
             raise RuntimeError('bqq_b200: rms_weight and swiglu cannot be combined')
@@ -401,23 +424,9 @@ class _BqqForwardMixin:
             nbytes = lib.bqq_forward_host_workspace_bytes(st.dims, M, code, code)
             ws = _workspace(device, 'host_decode' if M <= _cabi.DECODE_MAX_M else 'host_prefill', nbytes)
             stream = torch.cuda.current_stream(device).cuda_stream
-        args = (layer, x2.data_ptr(), code, M, x2.stride(0), y2.data_ptr(), code, y2.stride(0),
-                ws.data_ptr(), ws.numel(), stream)
-        call = lib.bqq_forward_host
-        index = device.index
-        keep = (x2, y2, ws, layer, st)                  # keeps the bound memory alive with the closure
-        result = out
-
-        def run():
-            if torch.cuda.current_device() != index:
-                with torch.cuda.device(index):
-                    rc = call(*args)
-            else:
-                rc = call(*args)
-            if rc:
-                check(rc, 'bqq_forward_host')
-            return result
-
+        keep = (layer, layer._keepalive, st)          # X_host stays the caller's to keep
+        run = _bqq_torch.make_host_call(C.addressof(layer), x2.data_ptr(), code, M, x2.stride(0), y2.data_ptr(), code,
+                                        y2.stride(0), ws.data_ptr(), ws.numel(), stream, device.index, out, keep)
         return run, out
 
     def forward_host(self, X_host, out=None):
@@ -431,6 +440,9 @@ class _BqqForwardMixin:
         return out
 
     def _weight_gpu(self, dtype):
+        W = _bqq_torch.weight(self.__dict__, _DTYPE_CODE[dtype])
+        if W is not None:
+            return W
         st = self._ensure_packed()
         device = st.zplanes.device
         out_f = self.row_width * self.y_row
@@ -477,6 +489,8 @@ class BinaryQuadratic(_BqqForwardMixin, nn.Module):
         self.c = nn.Parameter(coef[2].clone())
         self.d = nn.Parameter(coef[3].sum(dim=0))       # one offset per patch: summed over bit layers
         self.bias = nn.Parameter(bias) if bias is not None else None
+
+    _PLANE_SOURCES = ('Y', 'Z')
 
     def _plane_sources(self):
         return self.Y, self.Z
@@ -558,6 +572,8 @@ class PackedBinaryQuadratic(_BqqForwardMixin, nn.Module):
                    r, Y.shape[-2], Z.shape[-1],
                    bias=bq.bias.data.clone() if bq.bias is not None else None)
 
+    _PLANE_SOURCES = ('Y_packed', 'Z_packed')
+
     def _plane_sources(self):
         return self.Y_packed, self.Z_packed
 
@@ -630,6 +646,8 @@ class PlaneBinaryQuadratic(_BqqForwardMixin, nn.Module):
         return cls(zp, yp, coef[0].clone(), coef[1].clone(), coef[2].clone(), coef[3].sum(dim=0),
                    (bit_width, rw, cw, P, Q, r), bias=bias)
 
+    _PLANE_SOURCES = ('yplanes', 'zplanes')
+
     def _plane_sources(self):
         return self.yplanes, self.zplanes
 
@@ -649,6 +667,7 @@ class PlaneBinaryQuadratic(_BqqForwardMixin, nn.Module):
             st.zplanes, st.yplanes = self.zplanes.contiguous(), self.yplanes.contiguous()
             st.ysum = st.zsum = None
             st.plane_key = pkey
+            self._open_native(st)
         return st
 
     def get_weight(self, dtype=torch.float32):

@@ -1,8 +1,9 @@
-"""Build libbqq_b200.so (sm_100a) in-tree with nvcc.
+"""Build libbqq_b200.so (sm_100a) and the Python module's native side in-tree.
 
-Each .cu under csrc/ is compiled to an object file in parallel, then linked
-into bqq_b200/libbqq_b200.so.  Objects are rebuilt only when a source or header
-is newer.  Usable as `python -m bqq_b200.build [--force]`.
+Each .cu under csrc/ is compiled to an object file in parallel with nvcc, then linked
+into bqq_b200/libbqq_b200.so; csrc/bqq_torch.cpp becomes the extension module
+bqq_b200/_bqq_torch.so with g++ against the installed torch.  Objects are rebuilt only when
+a source or header is newer.  Usable as `python -m bqq_b200.build [--force]`.
 """
 from __future__ import annotations
 
@@ -18,6 +19,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, 'csrc')
 OBJ = os.path.join(PKG, 'build')
 LIB = os.path.join(PKG, 'libbqq_b200.so')
+EXT = os.path.join(PKG, '_bqq_torch.so')
 
 NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
               '-Xcompiler', '-fPIC', '-I' + os.path.join(ROOT, 'include'), '-I' + CSRC]
@@ -28,6 +30,21 @@ def nvcc_path() -> str:
     if not os.path.exists(exe):
         raise RuntimeError('nvcc not found; the bqq_b200 CUDA library cannot be built')
     return exe
+
+
+def _torch_command(src: str) -> list:
+    """g++ command of the extension module: linked against torch and, by its own folder, libbqq_b200.so."""
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(nvcc_path())), 'include')
+    inc = [os.path.join(base, 'include'), os.path.join(base, 'include', 'torch', 'csrc', 'api', 'include'), cuda,
+           sysconfig.get_paths()['include'], os.path.join(ROOT, 'include')]
+    return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared', '-fvisibility=hidden', '-w',
+            f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}', *('-I' + i for i in inc), src, '-o', EXT,
+            '-L' + os.path.join(base, 'lib'), '-L' + PKG, '-ltorch_python', '-ltorch', '-ltorch_cpu', '-ltorch_cuda',
+            '-lc10', '-lc10_cuda', '-l:libbqq_b200.so', '-Wl,-rpath,$ORIGIN']
 
 
 def _newest_header() -> float:
@@ -64,6 +81,12 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run([nvcc, '-shared', '-o', LIB, *objs], capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError('link failed:\n' + r.stdout + r.stderr)
+    src = os.path.join(CSRC, 'bqq_torch.cpp')
+    if force or not os.path.exists(EXT) or os.path.getmtime(EXT) < max(os.path.getmtime(src), os.path.getmtime(__file__),
+                                                                       _newest_header()):
+        cmd, r = run(_torch_command(src))
+        if r.returncode != 0:
+            raise RuntimeError('g++ failed: ' + ' '.join(cmd) + '\n' + r.stdout + r.stderr)
     return LIB
 
 
