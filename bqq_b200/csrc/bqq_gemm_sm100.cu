@@ -517,8 +517,8 @@ int prefill_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t
   auto rebuild = [&](int pnl, int pdl) {
     int i0, i1;
     panel_rows(pnl, &i0, &i1);
-    return f16 ? reconstruct_launch(L, W, nullptr, BQQ_F16, 1.f, bound_parts, st, i0, i1, pdl)
-               : reconstruct_launch(L, W, W + (size_t)N * K, BQQ_BF16, 1.f, nullptr, st, i0, i1, pdl);
+    return f16 ? reconstruct_launch(L, W, nullptr, BQQ_F16, 1.f, bound_parts, st, i0, i1, pdl, status)
+               : reconstruct_launch(L, W, W + (size_t)N * K, BQQ_BF16, 1.f, nullptr, st, i0, i1, pdl, status);
   };
   rc = rebuild(0, kPdlWaitFirst);
   if (rc) return rc;

@@ -1,0 +1,162 @@
+// One 32x32 block of the dense weight from its plane words, in registers:
+//   W[p][q] = sum_b ( a_b sum_k Y_b[p][k] Z_b[k][q] + b_b sum_k Y_b[p][k] + c_b sum_k Z_b[k][q] ) + d
+// by one warp.  Bound: issue and fixed-latency dependences of about 150 instructions per bit layer and 32 ranks at four
+// warps per scheduler (registers), with the int8 tensor pipe (14 products m16n8k32 of 9 clocks) about half busy; what is
+// not a product is kept as short as possible:
+//  * A count leaves the tensor core as an integer n 2^s (s: the powers of two that the operand masks below leave in).
+//    Its bit pattern, read as a float, IS the subnormal number n 2^(s-149), and a multiply-add takes subnormal inputs at
+//    full rate: with coefficients scaled by 2^84 the sums are ordinary floats of full precision, and one multiply-add
+//    per entry and bit layer is all there is - no conversion, no start value.  The powers of two are taken out once at
+//    the end.  (Coefficients beyond 2^43 would overflow; products below 2^-87 would lose bits.)
+//  * Y (A operand): a lane's plane word holds rows g + 8 rr and ranks 16 kh + 4 t + e at bit 8 e + 4 kh + rr, so
+//    word & (0x01010101 << rr) is an operand register (bytes 0 or 2^rr).
+//  * Z (B operand): the four ranks of one column are one nibble of a plane word.  byte * 0x08040201 repeats the byte
+//    at a pitch of 9 bits, so bit 3 of byte s is bit 3 - s of the low nibble and bit 7 of byte s that of the high one:
+//    one multiplication and two masks make the registers of two 8-column tiles (bytes 0 or 8 and 0 or 128).  The ranks
+//    come out in reverse, so the bytes of the Y word are reversed too (any common order of the contraction serves).
+//  * Row and column sums are products with an operand of ones.
+// Column order: the tile nt = 2 qh + x holds, at column n, q = 16 qh + 4 (n >> 1) + 2 x' + (n & 1) with x' = x, or
+// x ^ (n >> 2) where SWAP is set; a lane thus owns q = 16 qh + 4 t + {0..3} of every row, in two pairs (x = 0, 1).
+// Without SWAP the pairs are in order (8- or 16-byte global stores that fill 32-byte sectors); with SWAP the lanes t < 2
+// and t >= 2 write different halves of their four entries at a time, so that 4-byte stores into rows of 128
+// swizzled bytes touch every bank once.
+#pragma once
+#include "bqq_common.cuh"
+
+namespace bqq {
+
+__device__ __forceinline__ void mma_u8u8_zero(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+}
+__device__ __forceinline__ void mma_u8u8_add(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+constexpr int kCoefExp = 84;                         // coefficients come in multiplied by 2^84
+constexpr float kCoefScale = 19342813113834066795298816.f;
+// 2^(62 - e): takes the powers of two out of a sum (62 = 149 - 84 - 3)
+template <int E>
+__device__ __forceinline__ float rebuild_unscale() {
+  static_assert(62 - E > -126 && 62 - E < 127, "");
+  return __int_as_float((127 + 62 - E) << 23);
+}
+
+// Where a lane finds its Z bytes.
+struct RebuildLane {
+  uint32_t zsel[2];            // byte of tile x, zeros above it
+  int zfrom;                   // plane lane of rank half 0 (rank half 1: + 16)
+};
+template <bool SWAP>
+__device__ __forceinline__ RebuildLane rebuild_lane(int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  const uint32_t e = (SWAP ? 2 * (g >> 2) : 0) + (g & 1);
+  RebuildLane L;
+  L.zsel[0] = 0x4440u | e;
+  L.zsel[1] = 0x4440u | (e ^ 2u);
+  L.zfrom = 4 * t + (g >> 1);
+  return L;
+}
+
+// Sums of a block so far: acc[rr][nt] = rows g + 8 rr, two columns each; what depends on the row or on the column only is
+// kept apart until the end.
+struct RebuildAcc {
+  float2 acc[4][4];
+  float row[4];
+  float2 col[4];
+};
+// Takes the powers of two out of the row and column terms (d joins the rows) ...
+__device__ __forceinline__ void rebuild_end(RebuildAcc& r, float d) {
+  r.row[0] = fmaf(r.row[0], rebuild_unscale<0>(), d);
+  r.row[1] = fmaf(r.row[1], rebuild_unscale<1>(), d);
+  r.row[2] = fmaf(r.row[2], rebuild_unscale<2>(), d);
+  r.row[3] = fmaf(r.row[3], rebuild_unscale<3>(), d);
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    const float u = nt < 2 ? rebuild_unscale<0>() : rebuild_unscale<4>();
+    r.col[nt].x *= u;
+    r.col[nt].y *= u;
+  }
+}
+// ... and gives the entries of row g + 8 RR in tile NT: acc 2^(62-e) + (col + row), two at a time.
+template <int RR, int NT>
+__device__ __forceinline__ float2 rebuild_entry(const RebuildAcc& r) {
+  constexpr int E = RR + (NT < 2 ? 0 : 4);
+  unsigned long long v, t;
+  float2 o;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(r.col[NT].x), "f"(r.col[NT].y));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(t) : "f"(r.row[RR]));
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(t));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(t) : "f"(rebuild_unscale<E>()));
+  asm("{\n\t.reg .b64 a;\n\tmov.b64 a, {%1, %2};\n\tfma.rn.f32x2 %0, a, %3, %0;\n\t}"
+      : "+l"(v) : "f"(r.acc[RR][NT].x), "f"(r.acc[RR][NT].y), "l"(t));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(v));
+  return o;
+}
+
+template <bool FIRST>
+__device__ __forceinline__ void fma_pair(float2& acc, float k, int n0, int n1) {
+  acc.x = FIRST ? k * __int_as_float(n0) : fmaf(k, __int_as_float(n0), acc.x);
+  acc.y = FIRST ? k * __int_as_float(n1) : fmaf(k, __int_as_float(n1), acc.y);
+}
+
+// Adds one bit layer (FIRST: starts the sums with it).  y, z: the words of this lane's col patch in RT blocks of 32 lanes x 4 col patches of Y and of Z
+// (shared memory).
+template <int RT, bool FIRST>
+__device__ __forceinline__ void rebuild_bit(RebuildAcc& r, const RebuildLane& L, const uint32_t* y, const uint32_t* z,
+                                            int lane, float a, float b, float c) {
+  uint32_t A[RT][2][4], B[RT][4][2];
+#pragma unroll
+  for (int rt = 0; rt < RT; ++rt) {
+    const uint32_t w = __byte_perm(y[rt * 128 + lane * 4], 0u, 0x0123);
+    const uint32_t w4 = w >> 4;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+      A[rt][mt][0] = w & (0x01010101u << (2 * mt));
+      A[rt][mt][1] = w & (0x02020202u << (2 * mt));
+      A[rt][mt][2] = w4 & (0x01010101u << (2 * mt));
+      A[rt][mt][3] = w4 & (0x02020202u << (2 * mt));
+    }
+#pragma unroll
+    for (int kh = 0; kh < 2; ++kh) {
+      const uint32_t v = z[rt * 128 + (L.zfrom + 16 * kh) * 4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const uint32_t m = __byte_perm(v, 0u, L.zsel[x]) * 0x08040201u;
+        B[rt][x][kh] = m & 0x08080808u;
+        B[rt][2 + x][kh] = m & 0x80808080u;
+      }
+    }
+  }
+  const uint32_t ones[4] = {0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u};
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt) {                   // row sums: B = 8 everywhere
+    int d[4];
+    mma_u8u8_zero(d, A[0][mt], 0x08080808u, 0x08080808u);
+    if (RT == 2) mma_u8u8_add(d, A[RT - 1][mt], 0x08080808u, 0x08080808u);
+    r.row[2 * mt] = FIRST ? b * __int_as_float(d[0]) : fmaf(b, __int_as_float(d[0]), r.row[2 * mt]);
+    r.row[2 * mt + 1] = FIRST ? b * __int_as_float(d[2]) : fmaf(b, __int_as_float(d[2]), r.row[2 * mt + 1]);
+  }
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    int dc[4], d0[4], d1[4];
+    mma_u8u8_zero(dc, ones, B[0][nt][0], B[0][nt][1]);
+    mma_u8u8_zero(d0, A[0][0], B[0][nt][0], B[0][nt][1]);
+    mma_u8u8_zero(d1, A[0][1], B[0][nt][0], B[0][nt][1]);
+    if (RT == 2) {
+      mma_u8u8_add(dc, ones, B[RT - 1][nt][0], B[RT - 1][nt][1]);
+      mma_u8u8_add(d0, A[RT - 1][0], B[RT - 1][nt][0], B[RT - 1][nt][1]);
+      mma_u8u8_add(d1, A[RT - 1][1], B[RT - 1][nt][0], B[RT - 1][nt][1]);
+    }
+    fma_pair<FIRST>(r.col[nt], c, dc[0], dc[1]);
+    fma_pair<FIRST>(r.acc[0][nt], a, d0[0], d0[1]);
+    fma_pair<FIRST>(r.acc[1][nt], a, d0[2], d0[3]);
+    fma_pair<FIRST>(r.acc[2][nt], a, d1[0], d1[1]);
+    fma_pair<FIRST>(r.acc[3][nt], a, d1[2], d1[3]);
+  }
+}
+
+}  // namespace bqq

@@ -3,20 +3,26 @@
 //                             + c_b popc(Zcol_b[q]) ) + d
 // i.e. BinaryQuadratic.get_weight (neural_network_compression/src/bqq_modules.py:48-55); replaces
 // reconstruct_W_kernel (src/bqq_cuda.cu:198-246).
-// A warp owns one 32x32 block of one patch and forms the counts Y Z on the tensor cores
-// (mma.sync m16n8k16, fp16 operands that are 2.0 or zero, fp32 accumulators: the sums are exact).  The Y plane word of a lane is already an A fragment (rows of Y over the rank);
-// the Z plane word is a fragment over q whose four rows are four consecutive ranks, exactly the four
-// ranks a lane of the B fragment needs for one column: the lane fetches the words of four plane lanes
-// (four shuffles) and expands one nibble per rank half and 8-column tile.
-// Row and column sums come from two more products with an all-ones operand, so one bit layer costs
-// 28 MMAs, 44 FMAs and about 90 integer instructions per warp.
+// A compute warp forms one 32x32 block of one patch at a time with int8 tensor-core products (bqq_rebuild.cuh, where the
+// cost per bit layer is accounted for).  A stage of work is two super-groups at one block position: eight compute warps take
+// their eight col patches (the plane words of a super-group's four are interleaved).  A producer warp runs a few stages
+// ahead: it brings the plane words by bulk copies, the coefficients as floats and the place of the results, so that a step
+// of a compute warp (one block, one bit layer) is four shared-memory loads and the arithmetic.  Measured, 4096 x 14336
+// with 4 bit layers to bf16: 125.7 us with fp16 products, addresses and coefficients in every warp -> 64 us (53 us of
+// it without the stores); 45 % of the tensor pipe, 65 % of the issue slots, 2.8 TB/s.
 #include <algorithm>
+#include <type_traits>
 
-#include "bqq_common.cuh"
+#include "bqq_async.cuh"
+#include "bqq_rebuild.cuh"
 
 namespace bqq {
 
-constexpr int kReconWarps = 4;
+constexpr int kReconGroups = 2;                    // super-groups of a stage
+constexpr int kReconWarps = kReconGroups * kGroup; // compute warps
+constexpr int kReconThreads = (kReconWarps + 2) * 32;
+constexpr int kReconStages = 4;                    // stages in flight
+constexpr int kReconBits = 8;                      // bit layers of a stage at most
 
 struct ReconParams {
   const uint32_t* zp;
@@ -27,12 +33,14 @@ struct ReconParams {
   const float* bound_parts;    // optional: entries are also scaled by w_scale_from_bound
   float scale;
   int coef_dtype, w_dtype;
-  int pairs;                   // 1: two neighbouring entries of a row may be stored as one aligned word
+  int quads;                   // 1: four neighbouring entries of a row may be stored as one aligned word
   Geom g;
-  int tasks_per_row;           // cw * PT * QT: 32x32 blocks of one row patch
+  int units;                   // super-groups of these row patches
+  int step_i, step_jg;         // kReconGroups gridDim.x super-groups further: row patches and super-groups
   int i0, i1;                  // row patches [i0, i1) are rebuilt
   // How the launch takes part in a chain of programmatic dependent launches (kPdl* in bqq_common.cuh)
   int pdl;
+  unsigned* status;            // optional word, set when a wait on a copy gave up
 };
 
 // element type of W as a compile-time choice
@@ -59,267 +67,251 @@ template <> struct WType<BQQ_F16> {
   static __device__ __forceinline__ float back(T v) { return __half2float(v); }
 };
 
-// Bits POS + 8 ODD and POS + 8 ODD + 16 of w as two fp16 numbers, each 2.0 (0x4000) or zero: entries ODD and
-// ODD + 2 of the four consecutive ranks a plane word holds for one row (column) at in-byte position POS.
-template <int POS, int ODD>
-__device__ __forceinline__ uint32_t bits_as_half2(uint32_t w) {
-  constexpr int src = POS + 8 * ODD;
-  return (src <= 14 ? w << (14 - src) : w >> (src - 14)) & 0x40004000u;
+// four neighbouring entries as one 8- or 16-byte store
+__device__ __forceinline__ void store_quad(float* p, float2 a, float2 b) {
+  *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
 }
-constexpr uint32_t kOnesHalf2 = 0x3C003C00u;     // 1.0 twice
-constexpr float kBitValue = 2.0f;                // value of a set entry
-
-// D = A B (+ D): A 16x16 (rows g and g+8 of a lane), B 16x8 (column g), fp16 operands, fp32 accumulators.
-// The order of the 16 entries of k is the same in A and B, so any order serves.
-__device__ __forceinline__ void mma_f16_first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%10,%10,%10,%10};\n"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+template <typename T, typename T2>
+__device__ __forceinline__ void store_quad(T* p, T2 a, T2 b) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
 }
 
-// Fragments of rank half KH: rows g + 8 R0 and g + 8 (R0 + 1) of Y, entries {0, 2} and {1, 3} of the lane's ranks
-template <int KH, int R0>
-__device__ __forceinline__ void y_frag(uint32_t (&a)[4], uint32_t yw) {
-  a[0] = bits_as_half2<4 * KH + R0, 0>(yw);
-  a[1] = bits_as_half2<4 * KH + R0 + 1, 0>(yw);
-  a[2] = bits_as_half2<4 * KH + R0, 1>(yw);
-  a[3] = bits_as_half2<4 * KH + R0 + 1, 1>(yw);
-}
-// B fragment from a nibble m of a Z plane word: bits rr = 0..3 are Z[k0 + rr][q] for the four ranks of one lane of
-// the A fragment, whose k order is (0, 2 | 1, 3).  One multiplication moves bit 0 (1) to bit 14 and bit 2 (3) to
-// bit 30, the places where an fp16 pair reads 2.0; the other partial products fall outside the mask.
-__device__ __forceinline__ void z_frag(uint32_t (&b)[2], uint32_t m) {
-  b[0] = (m * 0x10004000u) & 0x40004000u;
-  b[1] = (m * 0x08002000u) & 0x40004000u;
-}
-
-// First word of Y and of Z (for the lane that reads plane lane `zsrc`) and first coefficient of one 32x32 block.
-struct ReconTask {
-  const uint32_t* y;
-  const uint32_t* z;
-  size_t ci;                   // i * cw + j
-  int i, j, pt, qt;
+// The stages of one group of a CTA, in order: super-groups u = 2 (blockIdx.x + k gridDim.x) + group of the row patches
+// [i0, i1) (counted row patch by row patch), their blocks, and up to kReconBits bit layers from bit0 at a time.
+struct ReconWalk {
+  int i, jg, pt, qt, bit0, u;
+  __device__ __forceinline__ void start(const ReconParams& p, int group) {
+    u = (int)blockIdx.x * kReconGroups + group;
+    i = p.i0 + u / p.g.JG;
+    jg = u % p.g.JG;
+    pt = qt = bit0 = 0;
+  }
+  __device__ __forceinline__ bool there(const ReconParams& p) const { return u < p.units; }
+  __device__ __forceinline__ void next(const ReconParams& p, int nb) {
+    bit0 += nb;
+    if (bit0 < p.g.bw) return;
+    bit0 = 0;
+    if (++qt < p.g.QT) return;
+    qt = 0;
+    if (++pt < p.g.PT) return;
+    pt = 0;
+    u += (int)gridDim.x * kReconGroups;
+    i += p.step_i;
+    jg += p.step_jg;
+    if (jg >= p.g.JG) { jg -= p.g.JG; ++i; }
+  }
+};
+// What a stage holds beside its plane words.
+struct ReconHead {
+  long long at;                // entry (0, 0) of the block of col patch 0 in W, in elements
+  int rows, cols;              // rows and columns of the block that exist
+  int patches;                 // col patches that exist (0: no super-group here)
+  int pad[3];
+};
+struct ReconStage {
+  ReconHead head[kReconGroups];
+  float4 coef[kReconGroups][kReconBits][kGroup];   // {a, b, c, d}
 };
 
-template <int RT>
-__device__ __forceinline__ ReconTask recon_locate(const ReconParams& p, int i, unsigned tj, int lane, int zsrc) {
-  const Geom& g = p.g;
-  ReconTask t;
-  t.i = i;
-  t.qt = 0; t.pt = 0; t.j = (int)tj;
-  if (g.PT * g.QT != 1) {
-    unsigned u = tj;
-    t.qt = (int)(u % (unsigned)g.QT); u /= (unsigned)g.QT;
-    t.pt = (int)(u % (unsigned)g.PT);
-    t.j = (int)(u / (unsigned)g.PT);
-  }
-  const int sub = t.j % kGroup;
-  const size_t sg0 = (size_t)i * g.NS + t.j / kGroup;
-  t.y = p.yp + ((sg0 * g.PT + t.pt) * RT * 32 + lane) * kGroup + sub;
-  t.z = p.zp + ((sg0 * RT * g.QT + t.qt) * 32 + zsrc) * kGroup + sub;
-  t.ci = (size_t)i * g.cw + t.j;
-  return t;
-}
-
 template <int RT, int DT, bool LO>
-__global__ void __launch_bounds__(kReconWarps * 32, 4)
+__global__ void __launch_bounds__(kReconThreads, 2)
 bqq_reconstruct_kernel(const ReconParams p) {
   using WT = typename WType<DT>::T;
   using WT2 = typename WType<DT>::T2;
+  extern __shared__ __align__(128) uint8_t rsm[];    // planes: [stage][group][bit][Y RT x 512 | Z RT x 512 bytes]
+  __shared__ uint64_t full[kReconStages], used[kReconStages];
+  __shared__ __align__(16) ReconStage stage[kReconStages];
+  constexpr int kBitBytes = RT * 1024;
   const Geom& g = p.g;
-  const int lane = threadIdx.x & 31;
-  const int g8 = lane >> 2, t4 = lane & 3;
-  pdl_enter(p.pdl);
-  const float scale = p.bound_parts ? p.scale * w_scale_from_bound(p.bound_parts, (float)(g.bw * g.r)) : p.scale;
-  const float s_core = scale / (kBitValue * kBitValue), s_sum = scale / kBitValue;
-  const size_t ldw = (size_t)g.cw * g.Q;
-  // Z word -> B fragments.  Plane lane 4 gz + tz holds, at bit 8e + 4qh + rr, Z[k = 4 gz + rr][q = 16 qh + 4 tz + e].
-  // Lane (n = g8, t = t4) of a B fragment needs, for rank half kh and 8-column tile nt = 2 qh + x, the ranks
-  // 16 kh + 4 t + rr of column q = 8 nt + n: the nibble at byte n & 3, half qh, of plane lane
-  // 16 kh + 4 t + 2 x + (n >> 2).  It reads the plane word of lane `lane` itself as its own Z word (zsrc = lane).
-  const int zsrc = lane;
-  const int zfrom = 4 * t4 + (g8 >> 2);               // + 16 kh + 2 x
-  const uint32_t zbyte = 0x4440u | (uint32_t)(g8 & 3);   // byte n & 3 into the low byte, zeros above
-  const size_t ystep = (size_t)g.JG * g.PT * RT * 32 * kGroup, zstep = (size_t)g.JG * RT * g.QT * 32 * kGroup;
-  const size_t cstep = (size_t)g.rw * g.cw;
-
-  // A warp walks blocks first, first + stride, ... of the layer (row patch i, block tj of the row patch); the
-  // plane words and coefficients of the next step, and at the end those of the next block, are fetched one step ahead.
-  const unsigned tpr = (unsigned)p.tasks_per_row;
-  const unsigned stride = gridDim.x * kReconWarps;
-  unsigned tj = blockIdx.x * kReconWarps + (threadIdx.x >> 5);
-  int i = (int)(tj / tpr);
-  tj -= (unsigned)i * tpr;
-  i += p.i0;
-  bool have = i < p.i1;
-  ReconTask cur = recon_locate<RT>(p, have ? i : 0, have ? tj : 0u, lane, zsrc);
-  uint32_t yw_n = 0u, zw_n = 0u;
-  float ca_n = 0.f, cb_n = 0.f, cc_n = 0.f, d_n = 0.f;
-  if (have) {
-    yw_n = cur.y[0];
-    zw_n = cur.z[0];
-    ca_n = load_as_float(p.a, cur.ci, p.coef_dtype);
-    cb_n = load_as_float(p.b, cur.ci, p.coef_dtype);
-    cc_n = load_as_float(p.c, cur.ci, p.coef_dtype);
-    d_n = load_as_float(p.d, cur.ci, p.coef_dtype);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nb = min(g.bw, kReconBits), nchunks = (g.bw + nb - 1) / nb;   // bit layers of a stage, stages of a block
+  const int blocks = g.PT * g.QT;
+  const int pairs = (p.units + kReconGroups - 1) / kReconGroups;
+  const int mine = ((int)blockIdx.x < pairs ? (pairs - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0);
+  const int nstages = mine * blocks * nchunks;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kReconStages; ++s) { mbar_init(full + s, 2); mbar_init(used + s, kReconWarps); }
+    mbar_init_fence();
   }
+  __syncthreads();
 
-  while (have) {
-    unsigned ntj = tj + stride;
-    int ni = i;
-    if (ntj >= tpr) {
-      const unsigned k = ntj / tpr;
-      ni += (int)k;
-      ntj -= k * tpr;
-    }
-    const bool have_next = ni < p.i1;
-    const ReconTask nxt = have_next ? recon_locate<RT>(p, ni, ntj, lane, zsrc) : cur;
-
-    float acc[2][4][4];          // [16-row tile][8-column tile][fragment entry]
-    float rowt[2][2];            // sum_b b_b popc(Yrow_b) of rows g8 (+8) of each 16-row tile
-    float colt[4][2];            // d + sum_b c_b popc(Zcol_b) of columns 2 t4 (+1) of each 8-column tile
-    const float dterm = d_n * scale;
+  if (warp == kReconWarps) {
+    // ---- producer of the plane words: one lane, a few stages ahead ---------------------------------------
+    if (lane == 0) {
+      ReconWalk w0, w1;
+      w0.start(p, 0);
+      w1.start(p, 1);
+      for (int n = 0; n < nstages; ++n) {
+        const int s = n % kReconStages;
+        if (n >= kReconStages) mbar_wait(used + s, (uint32_t)(n / kReconStages - 1) & 1u);
+        const int nbits = min(nb, g.bw - w0.bit0);
+        mbar_expect_tx(full + s, (uint32_t)(nbits * kBitBytes) * (w1.there(p) ? 2u : 1u));
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-      rowt[mt][0] = rowt[mt][1] = 0.f;
+        for (int grp = 0; grp < kReconGroups; ++grp) {
+          ReconWalk& w = grp ? w1 : w0;
+          if (w.there(p)) {
+            const size_t sg = (size_t)w.i * g.NS + (size_t)w.bit0 * g.JG + w.jg;
+            const uint32_t* y = p.yp + (sg * g.PT + w.pt) * (RT * 128);
+            const uint32_t* z = p.zp + (sg * RT * g.QT + w.qt) * 128;
+            uint8_t* dst = rsm + (size_t)((s * kReconGroups + grp) * nb) * kBitBytes;
+            for (int b = 0; b < nbits; ++b) {
+              bulk_load(dst, y, RT * 512, full + s);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[mt][nt][e] = 0.f;
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) colt[nt][0] = colt[nt][1] = dterm;
-
-    for (int b = 0; b < g.bw; ++b) {
-      const float ca = ca_n * s_core, cb = cb_n * s_sum, cc = cc_n * s_sum;
-      const bool more = b + 1 < g.bw;
-      if (more || have_next) {
-        const size_t ci = more ? cur.ci + (size_t)(b + 1) * cstep : nxt.ci;
-        ca_n = load_as_float(p.a, ci, p.coef_dtype);
-        cb_n = load_as_float(p.b, ci, p.coef_dtype);
-        cc_n = load_as_float(p.c, ci, p.coef_dtype);
-        if (!more) d_n = load_as_float(p.d, ci, p.coef_dtype);
-      }
-#pragma unroll
-      for (int rt = 0; rt < RT; ++rt) {
-        const uint32_t yw = yw_n;
-        uint32_t zw = zw_n;
-        if (rt + 1 < RT) {
-          yw_n = cur.y[(size_t)b * ystep + (size_t)(rt + 1) * 32 * kGroup];
-          zw_n = cur.z[(size_t)b * zstep + (size_t)(rt + 1) * g.QT * 32 * kGroup];
-        } else if (more) {
-          yw_n = cur.y[(size_t)(b + 1) * ystep];
-          zw_n = cur.z[(size_t)(b + 1) * zstep];
-        } else if (have_next) {
-          yw_n = nxt.y[0];
-          zw_n = nxt.z[0];
-        }
-        // fragments of both rank halves: 16-row tile mt holds rows g8 + 8 (2 mt + h), 8-column tile nt columns 8 nt + n
-        uint32_t a[2][2][4], bz[4][2][2];
-        y_frag<0, 0>(a[0][0], yw); y_frag<1, 0>(a[0][1], yw);
-        y_frag<0, 2>(a[1][0], yw); y_frag<1, 2>(a[1][1], yw);
-#pragma unroll
-        for (int kh = 0; kh < 2; ++kh)
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            const uint32_t byte = __byte_perm(__shfl_sync(0xffffffffu, zw, zfrom + 16 * kh + 2 * x), 0u, zbyte);
-            z_frag(bz[x][kh], byte & 0xFu);          // qh = 0: tile x
-            z_frag(bz[2 + x][kh], byte >> 4);        // qh = 1: tile 2 + x
+              for (int rt = 0; rt < RT; ++rt) bulk_load(dst + (RT + rt) * 512, z + rt * g.QT * 128, 512, full + s);
+              dst += kBitBytes;
+              y += (size_t)g.JG * g.PT * (RT * 128);
+              z += (size_t)g.JG * RT * g.QT * 128;
+            }
           }
-        // independent accumulation chains are interleaved: the second MMA of a chain waits for the first
-        float d0[4], d1[4], dz[4];
-        mma_f16_first(d0, a[0][0], kOnesHalf2, kOnesHalf2);                   // row sums
-        mma_f16_first(d1, a[1][0], kOnesHalf2, kOnesHalf2);
-        mma_f16(d0, a[0][1], kOnesHalf2, kOnesHalf2);
-        mma_f16(d1, a[1][1], kOnesHalf2, kOnesHalf2);
-        rowt[0][0] = fmaf(cb, d0[0], rowt[0][0]);
-        rowt[0][1] = fmaf(cb, d0[2], rowt[0][1]);
-        rowt[1][0] = fmaf(cb, d1[0], rowt[1][0]);
-        rowt[1][1] = fmaf(cb, d1[2], rowt[1][1]);
-        const uint32_t ones[4] = {kOnesHalf2, kOnesHalf2, kOnesHalf2, kOnesHalf2};
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          mma_f16_first(dz, ones, bz[nt][0][0], bz[nt][0][1]);                // column sums
-          mma_f16_first(d0, a[0][0], bz[nt][0][0], bz[nt][0][1]);
-          mma_f16_first(d1, a[1][0], bz[nt][0][0], bz[nt][0][1]);
-          mma_f16(dz, ones, bz[nt][1][0], bz[nt][1][1]);
-          mma_f16(d0, a[0][1], bz[nt][1][0], bz[nt][1][1]);
-          mma_f16(d1, a[1][1], bz[nt][1][0], bz[nt][1][1]);
-          colt[nt][0] = fmaf(cc, dz[0], colt[nt][0]);
-          colt[nt][1] = fmaf(cc, dz[1], colt[nt][1]);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            acc[0][nt][e] = fmaf(ca, d0[e], acc[0][nt][e]);
-            acc[1][nt][e] = fmaf(ca, d1[e], acc[1][nt][e]);
-          }
+          w.next(p, nb);
         }
       }
     }
+    pdl_enter(p.pdl);
+  } else if (warp == kReconWarps + 1) {
+    // ---- producer of coefficients and places -------------------------------------------------------------
+    // lane = (group, col patch, kind): its coefficient (kind 0, 1, 2: a, b, c of every bit layer of the stage; 3: d)
+    const int grp = lane >> 4, sub = (lane >> 2) & 3, kind = lane & 3;
+    const void* const base = kind == 0 ? p.a : kind == 1 ? p.b : kind == 2 ? p.c : p.d;
+    ReconWalk w;
+    w.start(p, grp);
+    float v[kReconBits];
+    auto load = [&](auto one) {                      // the coefficients of stage w
+      const int j = w.jg * kGroup + sub;
+      const bool there = w.there(p) && j < g.cw;
+      const size_t at = ((size_t)(kind < 3 ? w.bit0 * g.rw : 0) + w.i) * g.cw + j, step = (size_t)g.rw * g.cw;
+      const int count = !there ? 0 : kind < 3 ? min(nb, g.bw - w.bit0) : 1;
+#pragma unroll
+      for (int b = 0; b < kReconBits; ++b) {
+        if (b >= nb) break;
+        v[b] = b < count ? one(at + b * step) : 0.f;
+      }
+    };
+    auto coefficients = [&]() {
+      if (p.coef_dtype == BQQ_F32) load([&](size_t e) { return reinterpret_cast<const float*>(base)[e]; });
+      else load([&](size_t e) { return load_as_float(base, e, p.coef_dtype); });
+    };
+    coefficients();
+    pdl_enter(p.pdl);
+    const float scale = p.bound_parts ? p.scale * w_scale_from_bound(p.bound_parts, (float)(g.bw * g.r)) : p.scale;
+    const float cscale = kind < 3 ? scale * kCoefScale : scale;
+    for (int n = 0; n < nstages; ++n) {
+      const int s = n % kReconStages;
+      if (n >= kReconStages) mbar_wait(used + s, (uint32_t)(n / kReconStages - 1) & 1u);
+      float* dst = reinterpret_cast<float*>(&stage[s].coef[grp][0][sub]) + kind;
+#pragma unroll
+      for (int b = 0; b < kReconBits; ++b) {
+        if (b >= nb) break;
+        dst[b * kGroup * 4] = v[b] * cscale;
+      }
+      if ((lane & 15) == 0) {
+        ReconHead h;
+        h.at = ((long long)w.i * g.P + 32 * w.pt) * ((long long)g.cw * g.Q) + (long long)w.jg * kGroup * g.Q + 32 * w.qt;
+        h.rows = min(32, g.P - 32 * w.pt);
+        h.cols = min(32, g.Q - 32 * w.qt);
+        h.patches = w.there(p) ? min(kGroup, g.cw - w.jg * kGroup) : 0;
+        stage[s].head[grp] = h;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + s);
+      w.next(p, nb);
+      coefficients();
+    }
+  } else {
+    // ---- compute warps ---------------------------------------------------------------------------------
+    pdl_enter(p.pdl);
+    const int grp = warp / kGroup, sub = warp % kGroup;
+    const int g8 = lane >> 2, t4 = lane & 3;
+    const RebuildLane L = rebuild_lane<false>(lane);
+    const long long ldw = (long long)g.cw * g.Q;
+    const long long here = (long long)sub * g.Q + g8 * ldw + 4 * t4;   // the lane's first entry inside a block
+    RebuildAcc r;
+    float d = 0.f;
+    bool ok = true;
+    int s = 0, chunk = 0;
+    uint32_t phase = 0;
+    for (int n = 0; n < nstages; ++n) {
+      ok = ok && mbar_wait(full + s, phase);
+      const ReconStage& st = stage[s];
+      const ReconHead& h = st.head[grp];
+      const int nbits = min(nb, g.bw - chunk * nb);
+      const bool live = sub < h.patches;
+      if (live) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(rsm + (size_t)((s * kReconGroups + grp) * nb) * kBitBytes) + sub;
+        int b = 0;
+        if (chunk == 0) {
+          const float4 k = st.coef[grp][0][sub];
+          d = k.w;
+          rebuild_bit<RT, true>(r, L, w, w + RT * 128, lane, k.x, k.y, k.z);
+          b = 1;
+        }
+#pragma unroll 1
+        for (; b < nbits; ++b) {
+          const float4 k = st.coef[grp][b][sub];
+          rebuild_bit<RT, false>(r, L, w + b * (kBitBytes / 4), w + b * (kBitBytes / 4) + RT * 128, lane, k.x, k.y, k.z);
+        }
+      }
+      const long long at = h.at + here;
+      const int rows = h.rows, cols = h.cols;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(used + s);
+      if (++s == kReconStages) { s = 0; phase ^= 1u; }
+      if (++chunk < nchunks) continue;
+      chunk = 0;
+      if (!live) continue;
 
-    // 32 x 32 entries: a lane holds two neighbouring columns of rows g8 + 8 (2 mt + h) in every 8-column tile
-    const int row0 = 32 * cur.pt + g8, col0 = 32 * cur.qt + 2 * t4;
-    const size_t at0 = ((size_t)cur.i * g.P + row0) * ldw + (size_t)cur.j * g.Q + col0;
-    WT* wp = reinterpret_cast<WT*>(p.W) + at0;
-    WT* lp = LO ? reinterpret_cast<WT*>(p.W_lo) + at0 : nullptr;
-    const bool whole = p.pairs && 32 * cur.pt + 32 <= g.P && 32 * cur.qt + 32 <= g.Q;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const size_t roff = (size_t)(16 * mt + 8 * h) * ldw;
-        const bool row_ok = whole || row0 + 16 * mt + 8 * h < g.P;
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const float v0 = acc[mt][nt][2 * h] + rowt[mt][h] + colt[nt][0];
-          const float v1 = acc[mt][nt][2 * h + 1] + rowt[mt][h] + colt[nt][1];
-          WT* w = wp + roff + 8 * nt;
+      // 32 x 32 entries: a lane holds four neighbouring columns of rows g8 + 8 rr in either half
+      rebuild_end(r, d);
+      WT* wp = reinterpret_cast<WT*>(p.W) + at;
+      WT* lp = LO ? reinterpret_cast<WT*>(p.W_lo) + at : nullptr;
+      const bool whole = p.quads && rows == 32 && cols == 32;
+      auto row = [&](auto RR) {
+        constexpr int rr = decltype(RR)::value;
+        auto half = [&](int qh, float2 v01, float2 v23) {
+          WT* w = wp + 8 * rr * ldw + 16 * qh;
+          WT* lo = LO ? lp + 8 * rr * ldw + 16 * qh : nullptr;
           if (whole) {
-            const WT2 wv = WType<DT>::cvt2(v0, v1);
-            *reinterpret_cast<WT2*>(w) = wv;
+            const WT2 w01 = WType<DT>::cvt2(v01.x, v01.y), w23 = WType<DT>::cvt2(v23.x, v23.y);
+            store_quad(w, w01, w23);
             if (LO)
-              *reinterpret_cast<WT2*>(lp + roff + 8 * nt) =
-                  WType<DT>::cvt2(v0 - WType<DT>::back(wv.x), v1 - WType<DT>::back(wv.y));
-          } else if (row_ok) {
-            const int col = col0 + 8 * nt;
-            if (col < g.Q) {
-              const WT w0 = WType<DT>::cvt(v0);
-              w[0] = w0;
-              if (LO) lp[roff + 8 * nt] = WType<DT>::cvt(v0 - WType<DT>::back(w0));
-            }
-            if (col + 1 < g.Q) {
-              const WT w1 = WType<DT>::cvt(v1);
-              w[1] = w1;
-              if (LO) lp[roff + 8 * nt + 1] = WType<DT>::cvt(v1 - WType<DT>::back(w1));
-            }
+              store_quad(lo, WType<DT>::cvt2(v01.x - WType<DT>::back(w01.x), v01.y - WType<DT>::back(w01.y)),
+                         WType<DT>::cvt2(v23.x - WType<DT>::back(w23.x), v23.y - WType<DT>::back(w23.y)));
+          } else if (g8 + 8 * rr < rows) {
+            const float v[4] = {v01.x, v01.y, v23.x, v23.y};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (4 * t4 + 16 * qh + e < cols) {
+                const WT t = WType<DT>::cvt(v[e]);
+                w[e] = t;
+                if (LO) lo[e] = WType<DT>::cvt(v[e] - WType<DT>::back(t));
+              }
           }
-        }
-      }
-
-    cur = nxt;
-    i = ni;
-    tj = ntj;
-    have = have_next;
+        };
+        half(0, rebuild_entry<rr, 0>(r), rebuild_entry<rr, 1>(r));
+        half(1, rebuild_entry<rr, 2>(r), rebuild_entry<rr, 3>(r));
+      };
+      row(std::integral_constant<int, 0>());
+      row(std::integral_constant<int, 1>());
+      row(std::integral_constant<int, 2>());
+      row(std::integral_constant<int, 3>());
+    }
+    if (!ok && p.status && lane == 0) atomicExch(p.status, 1u);   // a bounded wait gave up: the entries are invalid
   }
   pdl_exit(p.pdl);
 }
 
 template <typename K>
 static int recon_launch_one(K kern, const ReconParams& p, dim3 blocks, cudaStream_t st) {
+  const size_t smem = (size_t)kReconStages * kReconGroups * std::min(p.g.bw, kReconBits) * p.g.RT * 1024;
+  if (smem > 32 * 1024 &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return BQQ_ERR_CUDA;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = blocks;
-  cfg.blockDim = dim3(kReconWarps * 32);
+  cfg.blockDim = dim3(kReconThreads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = p.pdl != kPdlNone ? 1 : 0;
@@ -339,22 +331,26 @@ static int reconstruct_dispatch(const ReconParams& p, dim3 blocks, cudaStream_t 
 }
 
 int reconstruct_launch(const BqqLayer* L, void* W, void* W_lo, int w_dtype, float scale, const float* bound_parts,
-                       cudaStream_t st, int i0, int i1, int pdl) {
+                       cudaStream_t st, int i0, int i1, int pdl, unsigned* status) {
   ReconParams p;
   p.g = Geom(L->dims);
   p.i0 = i0;
   p.i1 = i1 < 0 ? p.g.rw : i1;
   p.pdl = pdl;
+  p.status = status;
   p.zp = L->zplanes; p.yp = L->yplanes;
   p.a = L->a; p.b = L->b; p.c = L->c; p.d = L->d; p.coef_dtype = L->coef_dtype;
   p.W = W; p.W_lo = W_lo; p.scale = scale; p.bound_parts = bound_parts; p.w_dtype = w_dtype;
-  p.tasks_per_row = p.g.cw * p.g.PT * p.g.QT;      // in_features <= 2^30 keeps this far below 2^31
-  const uintptr_t pair_mask = 2 * (uintptr_t)dtype_size(w_dtype) - 1;
-  p.pairs = (p.g.Q % 2 == 0 && ((uintptr_t)W & pair_mask) == 0 && ((uintptr_t)W_lo & pair_mask) == 0) ? 1 : 0;
-  // resident warps walk the blocks: 4 CTAs per SM on 148 SMs
-  const long long tasks = (long long)p.tasks_per_row * (p.i1 - p.i0);
-  if (tasks <= 0) return BQQ_OK;
-  const dim3 blocks((unsigned)std::min<long long>((tasks + kReconWarps - 1) / kReconWarps, 148LL * 4));
+  const uintptr_t quad_mask = 4 * (uintptr_t)dtype_size(w_dtype) - 1;
+  p.quads = (p.g.Q % 4 == 0 && ((uintptr_t)W & quad_mask) == 0 && ((uintptr_t)W_lo & quad_mask) == 0) ? 1 : 0;
+  // resident CTAs walk the pairs of super-groups: 2 per SM on 148 SMs
+  const long long units = (long long)p.g.JG * (p.i1 - p.i0);
+  if (units <= 0) return BQQ_OK;
+  if (units > (1ll << 30)) return BQQ_ERR_UNSUPPORTED;
+  p.units = (int)units;
+  const dim3 blocks((unsigned)std::min<long long>((units + kReconGroups - 1) / kReconGroups, 148LL * 2));
+  p.step_i = (int)(blocks.x * kReconGroups) / p.g.JG;
+  p.step_jg = (int)(blocks.x * kReconGroups) % p.g.JG;
   if (w_dtype == BQQ_F32 && W_lo) return BQQ_ERR_UNSUPPORTED;     // a second part only exists for 16-bit types
   if (p.g.RT == 1) return reconstruct_dispatch<1>(p, blocks, st);
   return reconstruct_dispatch<2>(p, blocks, st);
