@@ -163,6 +163,7 @@ int decode_launch(const BqqLayer* layer, const void* x, int x_dtype, int M, int6
                   void* gathered = nullptr, int64_t ld_gathered = 0);   // with `peer`: the gathered rows [M, world * out]
 size_t peer_half_bytes(size_t gather_bytes);   // bytes of one half of a peer region's slot area
 size_t decode_workspace_bytes(const BqqDims* dims, int M);
+size_t decode_min_workspace_bytes(const BqqDims* dims, int M);   // what a call can do with at least
 constexpr size_t kPeerCtrlBytes = 512;   // control words at the start of a peer gather region (bqq_peer.cu)
 
 int decode_launches(const BqqDims* dims, int M);   // kernels per decode call: 1 or 2
@@ -171,6 +172,12 @@ size_t decode_counter_bytes();   // leading part of the decode workspace that mu
 int reconstruct_launch(const BqqLayer* layer, void* W, void* W_lo, int w_dtype, float scale,
                        const float* bound_parts, cudaStream_t stream, int i0 = 0, int i1 = -1, int pdl = kPdlNone,
                        unsigned* status = nullptr);   // status: word set when a bounded wait gave up
+// fused rebuild and multiply (bqq_fused.cu); counters: fused_counter_words() words that are zero unless `clear`
+constexpr int kFusedMaxM = 128;
+size_t fused_workspace_bytes(const Geom& g, int M);    // 0: not for this many rows
+size_t fused_counter_words(const Geom& g);
+int fused_launch(const BqqLayer* layer, const void* x, int x_dtype, int M, int64_t ldx, void* y, int y_dtype, int64_t ldy,
+                 unsigned* counters, unsigned* status, bool clear, void* scratch, const BqqFusion* fusion, cudaStream_t stream);
 int coef_bound_launch(const BqqLayer* layer, float* bound_parts, cudaStream_t stream);   // bound_parts zero on entry
 int prefill_launch(const BqqLayer* layer, const void* x, int x_dtype, int M, int64_t ldx, void* y,
                    int y_dtype, int64_t ldy, void* ws, size_t ws_bytes, cudaStream_t stream);

@@ -64,8 +64,23 @@ static DecodePlan make_decode_plan(const Geom& g, int M) {
 
 size_t decode_counter_bytes() { return kCounterBytes; }
 
+// The fused rebuild-and-multiply route costs the same for 2 and for 16 rows, the decode kernel about 12 us + 23 us per four
+// rows (4096 x 14336, 3 bit layers: 36 / 58 / 81 / 104 us against 75 us).  It is taken where it is the faster one: with 13
+// rows or more of 32x32 patches (larger patches share operands in the decode kernel, 22 against 27 us at 16 rows of
+// 4096 x 4096, P = Q = 64), and wherever the patch geometry runs in a decode variant with half as many blocks again as it
+// has (P = 96, Q = 40, r = 33: 23 against 19 us at 5 rows).  The rule knows nothing of the number of row patches, so a
+// row shard takes the route of the whole layer.
+static bool fused_decode(const Geom& g, int M) {
+  int v = 0;
+  while (v < 3 && !(g.PT <= kVariantPT[v] && g.QT <= kVariantQT[v] && g.RT <= kVariantRT[v])) ++v;
+  const int padded = kVariantRT[v] * (kVariantPT[v] + kVariantQT[v]), own = g.RT * (g.PT + g.QT);
+  const bool faster = g.PT * g.QT * g.RT == 1 ? M >= 13 : M >= 2 && 2 * padded >= 3 * own;
+  return faster && fused_counter_words(g) < (size_t)kMaxCounters && fused_workspace_bytes(g, M) > 0;
+}
+
 int decode_launches(const BqqDims* dims, int M) {
   Geom g(*dims);
+  if (fused_decode(g, M)) return g.Q == 32 ? 1 : 2;
   DecodePlan pl = make_decode_plan(g, M);
   if (pl.variant < 0) return BQQ_ERR_UNSUPPORTED;
   return pl.self_prep ? 1 : 2;
@@ -75,7 +90,26 @@ size_t decode_workspace_bytes(const BqqDims* dims, int M) {
   Geom g(*dims);
   DecodePlan pl = make_decode_plan(g, M);
   if (pl.variant < 0) return 0;
+  const size_t need = pl.xdig_bytes + pl.xmeta_bytes + align_up(pl.partial_floats * 4, 256);
+  return kCounterBytes + (fused_decode(g, M) ? std::max(need, fused_workspace_bytes(g, M)) : need);
+}
+// what the decode kernel itself needs: enough for a call that cannot have more
+size_t decode_min_workspace_bytes(const BqqDims* dims, int M) {
+  Geom g(*dims);
+  DecodePlan pl = make_decode_plan(g, M);
+  if (pl.variant < 0) return 0;
   return kCounterBytes + pl.xdig_bytes + pl.xmeta_bytes + align_up(pl.partial_floats * 4, 256);
+}
+
+// argument checks of a gathered call whose gather is a kernel of its own
+static int gather_check(const BqqPeerGroup* peer, int y_dtype, int M, int64_t n, const void* gathered, int64_t ld, int segments) {
+  if (!gathered) return BQQ_ERR_NULL;
+  const int64_t es = dtype_size(y_dtype);
+  if (segments > 2) return BQQ_ERR_UNSUPPORTED;
+  if (segments == 2 && (n * es) % 8) return BQQ_ERR_MISALIGNED;
+  if ((n * es) % 4 || (ld * es) % 4 || ((uintptr_t)gathered & 3)) return BQQ_ERR_MISALIGNED;
+  if ((uint64_t)M * n * peer->world * es > peer->gather_bytes) return BQQ_ERR_WORKSPACE;
+  return BQQ_OK;
 }
 
 int decode_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t ldx, void* y,
@@ -87,6 +121,27 @@ int decode_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t 
   if (pl.variant < 0) return BQQ_ERR_UNSUPPORTED;
   if ((size_t)g.rw * pl.mtiles > (size_t)kMaxCounters - 1) return BQQ_ERR_UNSUPPORTED;   // last word: status
   if ((size_t)g.bw * g.rw * g.cw >= (1ull << 31)) return BQQ_ERR_UNSUPPORTED;           // 32-bit coefficient offsets
+  if (!ws || ws_bytes < decode_min_workspace_bytes(&L->dims, M)) return BQQ_ERR_WORKSPACE;
+  if (((uintptr_t)ws & 255) != 0) return BQQ_ERR_MISALIGNED;
+  if (fused_decode(g, M) && ws_bytes >= kCounterBytes + fused_workspace_bytes(g, M)) {
+    if (peer) {
+      const int rc = gather_check(peer, y_dtype, M, g.out_features(), gathered, ld_gathered, fusion ? fusion->out_segments : 0);
+      if (rc) return rc;
+    }
+    unsigned* counters = reinterpret_cast<unsigned*>(ws);
+    const int rc = fused_launch(L, x, x_dtype, M, ldx, y, y_dtype, ldy, counters, counters + kMaxCounters - 1, false,
+                                reinterpret_cast<char*>(ws) + kCounterBytes, fusion, st);
+    if (rc || !peer) return rc;
+    // the sums of a tile are complete only in the CTA that finishes it last: the gather is a kernel of its own here
+    const int segments = fusion && fusion->out_segments == 2 ? 2 : 1;
+    const int64_t n = g.out_features() / segments;
+    for (int k = 0; k < segments; ++k) {
+      const int rg = bqq_peer_gather(peer, reinterpret_cast<const char*>(y) + k * n * dtype_size(y_dtype), y_dtype, M, n, ldy,
+                                     reinterpret_cast<char*>(gathered) + k * n * peer->world * dtype_size(y_dtype), ld_gathered, st);
+      if (rg) return rg;
+    }
+    return BQQ_OK;
+  }
   DecodeParams p;
   p.zp = reinterpret_cast<const uint4*>(L->zplanes);
   p.yp = reinterpret_cast<const uint4*>(L->yplanes);
@@ -97,9 +152,6 @@ int decode_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t 
   p.M = M; p.bw = g.bw; p.rw = g.rw; p.cw = g.cw; p.P = g.P; p.Q = g.Q;
   p.PTg = g.PT; p.QTg = g.QT; p.RTg = g.RT; p.JG = g.JG; p.NS = g.NS;
   p.sgw = pl.sgw; p.bpc = pl.bpc; p.nchunks = pl.nchunks; p.mtiles = pl.mtiles;
-  const size_t need = decode_workspace_bytes(&L->dims, M);
-  if (!ws || ws_bytes < need) return BQQ_ERR_WORKSPACE;
-  if (((uintptr_t)ws & 255) != 0) return BQQ_ERR_MISALIGNED;
   char* wsb = reinterpret_cast<char*>(ws);
   p.counters = reinterpret_cast<unsigned*>(wsb);
   p.xdig = reinterpret_cast<const uint8_t*>(wsb + kCounterBytes);

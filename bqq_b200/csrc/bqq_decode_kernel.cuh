@@ -43,6 +43,7 @@
 #pragma once
 #include "bqq_async.cuh"
 #include "bqq_common.cuh"
+#include "bqq_xsource.cuh"
 
 namespace bqq {
 
@@ -202,94 +203,6 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // (row, col patch) pair per 8 lanes.  `live` pairs read x[m, j*Q ...]; the others write zeros.
 // Digits go to words[] at the pair's place (M tile `mtile`, row `beta` inside it), statistics to
 // index `stat` of xscale / xsum / xl1.  Every lane of the warp must call it (shuffles).
-// Where the activation comes from, and what is applied to it on the way in (BqqFusion::prologue):
-// nothing, RMS normalisation (x * inv_rms * w[n]; inv_rms of the row is computed by the caller of
-// xprep_pair), or SwiGLU (silu(x[n]) * x[n + n_in], x holding [gate | up] rows of 2 * n_in elements).
-struct XSource {
-  const void* x;
-  const void* w;
-  int64_t ld;
-  int dtype, w_dtype, mode, n_in;
-  float eps;
-};
-__device__ __forceinline__ float load_x(const XSource& s, int m, int n, float inv_rms) {
-  float v = load_as_float(s.x, (size_t)m * s.ld + n, s.dtype);
-  if (s.mode == BQQ_PRO_RMSNORM) {
-    v = v * inv_rms * load_as_float(s.w, n, s.w_dtype);
-  } else if (s.mode == BQQ_PRO_SWIGLU) {
-    const float u = load_as_float(s.x, (size_t)m * s.ld + s.n_in + n, s.dtype);
-    v = v / (1.f + __expf(-v)) * u;
-  }
-  return v;
-}
-// Four consecutive elements n0 .. n0+3 of a tensor of type `dt` as floats; one 8- or 16-byte load when the
-// address allows it, four element loads otherwise.
-__device__ __forceinline__ void load_quad(const void* base, size_t idx, int dt, float (&v)[4]) {
-  if (dt == BQQ_F32) {
-    const float* p = reinterpret_cast<const float*>(base) + idx;
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-      const float4 q = *reinterpret_cast<const float4*>(p);
-      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = p[e];
-    }
-    return;
-  }
-  const uint16_t* p = reinterpret_cast<const uint16_t*>(base) + idx;
-  uint32_t w0, w1;
-  if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
-    const uint2 q = *reinterpret_cast<const uint2*>(p);
-    w0 = q.x; w1 = q.y;
-  } else {
-    w0 = (uint32_t)p[0] | ((uint32_t)p[1] << 16);
-    w1 = (uint32_t)p[2] | ((uint32_t)p[3] << 16);
-  }
-  if (dt == BQQ_BF16) {
-    v[0] = __uint_as_float(w0 << 16); v[1] = __uint_as_float(w0 & 0xFFFF0000u);
-    v[2] = __uint_as_float(w1 << 16); v[3] = __uint_as_float(w1 & 0xFFFF0000u);
-  } else {
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w0));
-    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&w1));
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
-}
-// x[m, n0 .. n0+3] after the prologue (all four columns exist)
-__device__ __forceinline__ void load_x_quad(const XSource& s, int m, int n0, float inv_rms, float (&v)[4]) {
-  load_quad(s.x, (size_t)m * s.ld + n0, s.dtype, v);
-  if (s.mode == BQQ_PRO_RMSNORM) {
-    float w[4];
-    load_quad(s.w, n0, s.w_dtype, w);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = v[e] * inv_rms * w[e];
-  } else if (s.mode == BQQ_PRO_SWIGLU) {
-    float u[4];
-    load_quad(s.x, (size_t)m * s.ld + s.n_in + n0, s.dtype, u);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = v[e] / (1.f + __expf(-v[e])) * u[e];
-  }
-}
-// Sum of squares of row m over this thread's share of the columns (threads tid, tid + n, ...).
-__device__ __forceinline__ float row_sumsq_share(const XSource& s, int m, int tid, int nthreads) {
-  float acc = 0.f;
-  if ((s.n_in & 3) == 0) {
-    for (int n = 4 * tid; n < s.n_in; n += 4 * nthreads) {
-      float v[4];
-      load_quad(s.x, (size_t)m * s.ld + n, s.dtype, v);
-      acc = fmaf(v[0], v[0], acc); acc = fmaf(v[1], v[1], acc);
-      acc = fmaf(v[2], v[2], acc); acc = fmaf(v[3], v[3], acc);
-    }
-  } else {
-    for (int n = tid; n < s.n_in; n += nthreads) {
-      const float v = load_as_float(s.x, (size_t)m * s.ld + n, s.dtype);
-      acc = fmaf(v, v, acc);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  return acc;                                       // the warp's share, in every lane
-}
-
 // `jsrc` is the col patch whose x is read, `j` its place in the output (they differ when a CTA prepares only
 // its own chunk: j counts from the chunk's first col patch, a multiple of 4).
 template <int QT>

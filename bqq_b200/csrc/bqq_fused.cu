@@ -1,0 +1,256 @@
+// Host side of the fused rebuild-and-multiply forward (algorithm and kernel in bqq_fused_kernel.cuh): plan, preparation of
+// x, launch.
+#include <algorithm>
+#include <type_traits>
+
+#include "bqq_fused_kernel.cuh"
+#include "bqq_xsource.cuh"
+
+namespace bqq {
+
+// x in the kernel's column order, zeros in the padding; also clears the counters of the tiles for callers whose scratch is not
+// kept clean.  Eight columns per thread.  NP (formats of bqq_fused_kernel.cuh) = 1: fp16, bf16 rows scaled by a power of
+// two (the row's maximum maps to at most 2^14; unscale[m] = 1 / scale); 2: bf16; 3: bf16 hi and lo = the rest.
+template <int NP>
+__global__ void __launch_bounds__(256)
+fused_prep_kernel(const XSource xs, int M, Geom g, int Kp, uint16_t* __restrict__ hi, uint16_t* __restrict__ lo,
+                  float* __restrict__ unscale, unsigned* __restrict__ zero, int nzero, unsigned* __restrict__ status) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (blockIdx.x == 0 && blockIdx.y == 0) {
+    for (int e = threadIdx.x; e < nzero; e += 256) zero[e] = 0u;
+    if (status && threadIdx.x == 0) *status = 0u;
+  }
+  if (!hi) return;
+  const int m = blockIdx.y;
+  __shared__ float part[8];
+  float inv_rms = 1.f, scale = 1.f;
+  if (NP != 1 && xs.mode == BQQ_PRO_RMSNORM) {
+    const float w = row_sumsq_share(xs, m, threadIdx.x, 256);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = w;
+    __syncthreads();
+    float tot = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) tot += part[k];
+    inv_rms = rsqrtf(tot / (float)xs.n_in + xs.eps);
+  }
+  if (NP == 1 && unscale) {
+    float top = 0.f;
+    if ((xs.n_in & 3) == 0) {
+      for (int n = 4 * threadIdx.x; n < xs.n_in; n += 1024) {
+        float v[4];
+        load_quad(xs.x, (size_t)m * xs.ld + n, xs.dtype, v);
+        top = fmaxf(top, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+      }
+    } else {
+      for (int n = threadIdx.x; n < xs.n_in; n += 256) top = fmaxf(top, fabsf(load_as_float(xs.x, (size_t)m * xs.ld + n, xs.dtype)));
+    }
+#pragma unroll
+    for (int e = 16; e > 0; e >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, e));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = top;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) top = fmaxf(top, part[k]);
+    const float parts[2] = {0.f, top};
+    scale = w_scale_from_bound(parts, 0.f);
+    if (threadIdx.x == 0 && blockIdx.x == 0) unscale[m] = 1.f / scale;
+  }
+  for (int k0 = (blockIdx.x * 256 + threadIdx.x) * 8; k0 < Kp; k0 += gridDim.x * 2048) {
+    const int blk = k0 >> 5, c0 = k0 & 31;
+    const int sub = blk & 3, s = blk >> 2;
+    const int jg = s / g.QT, qt = s - jg * g.QT;
+    const int j = jg * kGroup + sub, q = 32 * qt + c0;
+    float v[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float quad[4] = {0.f, 0.f, 0.f, 0.f};
+      if (j < g.cw && q + 4 * h + 4 <= g.Q) {
+        load_x_quad(xs, m, j * g.Q + q + 4 * h, inv_rms, quad);
+      } else if (j < g.cw) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (q + 4 * h + e < g.Q) quad[e] = load_x(xs, m, j * g.Q + q + 4 * h + e, inv_rms);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[4 * h + e] = quad[e];
+    }
+    uint32_t wh[4], wl[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (NP == 1) {
+        const __half2 b = __floats2half2_rn(v[2 * e] * scale, v[2 * e + 1] * scale);
+        wh[e] = *reinterpret_cast<const uint32_t*>(&b);
+        continue;
+      }
+      const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+      wh[e] = *reinterpret_cast<const uint32_t*>(&b);
+      const __nv_bfloat162 r = __floats2bfloat162_rn(v[2 * e] - __uint_as_float(wh[e] << 16),
+                                                     v[2 * e + 1] - __uint_as_float(wh[e] & 0xFFFF0000u));
+      wl[e] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    *reinterpret_cast<uint4*>(hi + (size_t)m * Kp + k0) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+    if (NP == 3) *reinterpret_cast<uint4*>(lo + (size_t)m * Kp + k0) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+  }
+}
+
+namespace {
+
+struct FusedPlan {
+  bool ok;
+  int N, nb, ns, nx, nw, tiles, chunks, chunk_stages, stages, Kp;
+  size_t smem, partial_bytes, x_bytes;
+};
+
+constexpr size_t kMaxSmem = 227 * 1024;
+inline size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+FusedPlan make_plan(const Geom& g, int M, int NP, bool any_rows) {
+  FusedPlan pl = {};
+  pl.N = (M + 15) / 16 * 16;
+  if (pl.N > (NP == 3 ? 64 : kFusedMaxN)) return pl;
+  const int RT = g.RT;
+  // Shared memory: at least two of everything, with as many bit layers per plane stage as that leaves room for; then deeper
+  // rings while there is room.  x first (a round trip for x is longer than a stage), then W buffers (they let the
+  // rebuild run ahead while x is being prepared), then planes.
+  pl.nb = 0;
+  auto fits = [&](int nb, int ns, int nx, int nw) { return (size_t)FusedSmem(NP, RT, pl.N, nb, ns, nx, nw).total <= kMaxSmem; };
+  for (int nb = std::min(g.bw, kFusedBits / RT); nb >= 1 && !pl.nb; --nb) {
+    if (!fits(nb, 2, 2, 2)) continue;
+    pl.nb = nb;
+    pl.ns = pl.nx = pl.nw = 2;
+    for (bool more = true; more;) {
+      more = false;
+      if (pl.nx < 3 && fits(nb, pl.ns, pl.nx + 1, pl.nw)) { ++pl.nx; more = true; }
+      if (pl.ns < 3 && fits(nb, pl.ns + 1, pl.nx, pl.nw)) { ++pl.ns; more = true; }
+      if (pl.nw < 4 && fits(nb, pl.ns, pl.nx, pl.nw + 1)) { ++pl.nw; more = true; }
+      if (!more && pl.nx < 4 && fits(nb, pl.ns, pl.nx + 1, pl.nw)) { ++pl.nx; more = true; }
+      if (!more && pl.ns < kFusedMaxPlaneStages && fits(nb, pl.ns + 1, pl.nx, pl.nw)) { ++pl.ns; more = true; }
+    }
+    pl.smem = FusedSmem(NP, RT, pl.N, nb, pl.ns, pl.nx, pl.nw).total;
+  }
+  if (!pl.nb) return pl;
+  pl.stages = g.JG * g.QT;
+  pl.Kp = pl.stages * kFusedStageCols;
+  pl.tiles = (g.rw * g.PT + 3) / 4;
+  // Chunk length: the cheapest by estimated clocks - rounds of items over 148 SMs, each a fixed part and its stages, then
+  // the sum over the chunks by one CTA.  Up to 16 rows the sum must not depend on the number of rows of W (a row shard
+  // reproduces the whole layer bit for bit), so the estimate is made for 4096 rows there.
+  const long long tiles = any_rows ? 32 : pl.tiles;
+  long long best = -1;
+  for (int cs = 1; cs <= pl.stages; ++cs) {
+    const int chunks = (pl.stages + cs - 1) / cs;
+    if (chunks > 32) continue;
+    const long long rounds = (tiles * chunks + 147) / 148;
+    const long long item = 1000 + (chunks > 1 ? 25LL * pl.N : 8LL * pl.N) + (long long)cs * (g.bw * RT * 1200LL + 600);
+    const long long cost = rounds * item + (chunks > 1 ? 2500 + 16LL * chunks * M * ((tiles + 147) / 148) : 0);
+    if (best < 0 || cost < best) { best = cost; pl.chunk_stages = cs; pl.chunks = chunks; }
+  }
+  pl.partial_bytes = pl.chunks > 1 ? up256((size_t)pl.tiles * pl.chunks * pl.N * kFusedTile * 4) : 0;
+  pl.x_bytes = up256((size_t)M * pl.Kp * 2) + 1024;         // and the factors of the rows
+  pl.ok = true;
+  return pl;
+}
+
+template <int NP, int RT>
+int launch(const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap& my, const CUtensorMap& mz, const FusedParams& p, const FusedPlan& pl, cudaStream_t st) {
+  auto kern = bqq_fused_kernel<NP, RT>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess) return BQQ_ERR_CUDA;
+  cudaLaunchAttribute attr[1] = {pdl_attribute()};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min(pl.tiles * pl.chunks, 148));
+  cfg.blockDim = dim3(kFusedThreads);
+  cfg.dynamicSmemBytes = pl.smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, hi, lo, my, mz, p) != cudaSuccess) { cudaGetLastError(); return BQQ_ERR_CUDA; }
+  return launch_status();
+}
+
+}  // namespace
+
+// Scratch beyond the counters: the larger of the ways x may come in (0: not for this many rows).
+size_t fused_workspace_bytes(const Geom& g, int M) {
+  size_t need = 0;
+  for (int NP = 1; NP <= 3; ++NP) {
+    const FusedPlan pl = make_plan(g, M, NP, M <= BQQ_DECODE_MAX_M);
+    if (!pl.ok) continue;
+    need = std::max(need, pl.partial_bytes + (size_t)(NP == 3 ? 2 : 1) * pl.x_bytes);
+  }
+  return need;
+}
+size_t fused_counter_words(const Geom& g) { return ((size_t)g.rw * g.PT + 3) / 4; }
+
+int fused_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t ldx, void* y, int y_dtype, int64_t ldy,
+                 unsigned* counters, unsigned* status, bool clear, void* scratch, const BqqFusion* fusion, cudaStream_t st) {
+  const Geom g(L->dims);
+  const bool prologue = fusion && fusion->prologue != BQQ_PRO_NONE;
+  const int NP = x_dtype == BQQ_F32 || prologue ? 3 : M > BQQ_DECODE_MAX_M ? 1 : x_dtype == BQQ_BF16 ? 2 : 3;
+  const FusedPlan pl = make_plan(g, M, NP, M <= BQQ_DECODE_MAX_M);
+  if (!pl.ok) return BQQ_ERR_UNSUPPORTED;
+  uint8_t* sc = reinterpret_cast<uint8_t*>(scratch);
+  uint16_t* xhi = reinterpret_cast<uint16_t*>(sc + pl.partial_bytes);
+  uint16_t* xlo = reinterpret_cast<uint16_t*>(sc + pl.partial_bytes + pl.x_bytes);
+  float* unscale = reinterpret_cast<float*>(sc + pl.partial_bytes + pl.x_bytes - 1024);
+  // rows in the kernel's own format and column order are read where they are
+  const bool direct = x_dtype == (NP == 1 ? BQQ_F16 : BQQ_BF16) && NP != 3 && g.Q == 32 && ldx % 8 == 0 && ((uintptr_t)x & 15) == 0;
+
+  FusedParams p;
+  p.zp = L->zplanes; p.yp = L->yplanes;
+  p.a = L->a; p.b = L->b; p.c = L->c; p.d = L->d; p.bias = L->bias;
+  p.res = fusion ? fusion->residual : nullptr;
+  p.ld_res = fusion ? fusion->ld_residual : 0;
+  p.res_dtype = fusion ? fusion->residual_dtype : 0;
+  p.y = y; p.ldy = ldy; p.y_dtype = y_dtype;
+  p.partial = reinterpret_cast<float*>(sc);
+  p.counters = counters;
+  p.status = status;
+  p.coef_dtype = L->coef_dtype; p.bias_dtype = L->bias_dtype;
+  p.g = g;
+  p.M = M; p.N = pl.N;
+  p.nb = pl.nb; p.ns = pl.ns; p.nx = pl.nx; p.nw = pl.nw;
+  p.row_unscale = NP == 1 && x_dtype == BQQ_BF16 ? unscale : nullptr;
+  p.tiles = pl.tiles; p.chunks = pl.chunks; p.chunk_stages = pl.chunk_stages; p.stages = pl.stages;
+  // fp32 accumulators, both operands fp16 or bf16, K-major; M = 128, N rows of x
+  const uint32_t fmt = NP == 1 ? 0u : 1u;
+  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(pl.N >> 3) << 17) | (8u << 24);
+
+  p.joint = g.PT == 1 && pl.nb == g.bw;
+  CUtensorMap hi, lo, my, mz;
+  int rc = direct ? make_map(&hi, x, NP != 1, (uint64_t)M, (uint64_t)g.in_features(), (uint64_t)ldx, (uint32_t)pl.N)
+                  : make_map(&hi, xhi, NP != 1, (uint64_t)M, (uint64_t)pl.Kp, (uint64_t)pl.Kp, (uint32_t)pl.N);
+  if (rc) return rc;
+  if (NP == 3) {
+    rc = make_map(&lo, xlo, true, (uint64_t)M, (uint64_t)pl.Kp, (uint64_t)pl.Kp, (uint32_t)pl.N);
+    if (rc) return rc;
+  } else {
+    lo = hi;
+  }
+  rc = make_plane_maps(&my, &mz, g, L->yplanes, L->zplanes, (uint32_t)(p.joint ? 4 * pl.nb : pl.nb));
+  if (rc) return rc;
+  if (!direct || clear) {
+    const XSource xs = {x, fusion ? fusion->norm_weight : nullptr, ldx, x_dtype, fusion ? fusion->norm_dtype : 0,
+                        prologue ? fusion->prologue : BQQ_PRO_NONE, g.in_features(), fusion ? fusion->eps : 0.f};
+    cudaLaunchAttribute attr[1] = {pdl_attribute()};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = direct ? dim3(1) : dim3((unsigned)std::min((pl.Kp + 2047) / 2048, 64), (unsigned)M);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int nzero = clear ? pl.tiles : 0;
+    uint16_t* h = direct ? nullptr : xhi;
+    unsigned* stw = clear ? status : nullptr;
+    float* un = const_cast<float*>(p.row_unscale);
+    auto kern = NP == 1 ? fused_prep_kernel<1> : NP == 2 ? fused_prep_kernel<2> : fused_prep_kernel<3>;
+    if (cudaLaunchKernelEx(&cfg, kern, xs, M, g, pl.Kp, h, xlo, un, counters, nzero, stw) != cudaSuccess) {
+      cudaGetLastError();
+      return BQQ_ERR_CUDA;
+    }
+  }
+  if (NP == 1) return g.RT == 1 ? launch<1, 1>(hi, lo, my, mz, p, pl, st) : launch<1, 2>(hi, lo, my, mz, p, pl, st);
+  if (NP == 2) return g.RT == 1 ? launch<2, 1>(hi, lo, my, mz, p, pl, st) : launch<2, 2>(hi, lo, my, mz, p, pl, st);
+  return g.RT == 1 ? launch<3, 1>(hi, lo, my, mz, p, pl, st) : launch<3, 2>(hi, lo, my, mz, p, pl, st);
+}
+
+}  // namespace bqq

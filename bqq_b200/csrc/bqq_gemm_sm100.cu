@@ -22,10 +22,9 @@
 // GEMM tiles each): bound, rebuild panel 0, stage x, then alternately multiply panel p and rebuild
 // panel p+1.  A GEMM waits for everything before it and then lets the next rebuild start at once, so the
 // rebuild of a panel (ALU work) runs beside the GEMM of the previous one (TMA and tensor pipe).
-#include <cuda.h>
+#include <algorithm>
 
-#include "bqq_async.cuh"
-#include "bqq_common.cuh"
+#include "bqq_tc.cuh"
 
 namespace bqq {
 
@@ -33,48 +32,6 @@ constexpr int kBM = 128;
 constexpr int kBK = 64;          // 64 x 2 bytes = one 128-byte swizzle row
 constexpr int kGemmThreads = 192;
 __host__ __device__ constexpr int gemm_stages(int BN, int MT) { return (BN == 256 && MT == 2) ? 3 : 4; }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
-}
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes,
-// 128-byte swizzled, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);          // start address, 16-byte units
-  d |= (uint64_t)1 << 16;                              // leading byte offset (one 16-byte unit; unused by swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;                    // stride byte offset between 8-row groups
-  d |= (uint64_t)1 << 46;                              // descriptor version of this architecture
-  d |= (uint64_t)2 << 61;                              // 128-byte swizzle
-  return d;
-}
-
 struct GemmParams {
   void* y;
   const void* bias;
@@ -350,56 +307,17 @@ stage_x_bf16_to_f16_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int
 }
 
 // ---- host side -----------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
-// 2-D row-major [rows][cols] 16-bit tensor, box = box_rows x 64 columns, 128-byte swizzle.
-static int make_map(CUtensorMap* map, const void* ptr, bool bf16, uint64_t rows, uint64_t cols,
-                    uint64_t ld_elems, uint32_t box_rows) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return BQQ_ERR_CUDA;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld_elems * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                  const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? BQQ_OK : BQQ_ERR_CUDA;
-}
-
 static inline size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
 // workspace: [256 B: status word, bound parts at +16][W parts 2 x N x K 16-bit][x hi M x K][x lo M x K]
 size_t prefill_workspace_bytes(const BqqDims* dims, int M) {
   Geom g(*dims);
   const size_t K = g.in_features();
-  return 256 + up256((size_t)2 * g.out_features() * K * 2) + 2 * up256((size_t)M * K * 2);
+  const size_t need = 256 + up256((size_t)2 * g.out_features() * K * 2) + 2 * up256((size_t)M * K * 2);
+  if (M > kFusedMaxM) return need;
+  return std::max(need, 256 + up256(fused_counter_words(g) * 4) + fused_workspace_bytes(g, M));
 }
 
-
-static cudaLaunchAttribute pdl_attribute() {
-  cudaLaunchAttribute a;
-  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  a.val.programmaticStreamSerializationAllowed = 1;
-  return a;
-}
 
 // tiles [tile0, tile0 + ntiles) along N, all of M
 template <int BN, int MT>
@@ -437,7 +355,6 @@ int prefill_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t
                    int64_t ldy, void* ws, size_t ws_bytes, cudaStream_t st) {
   Geom g(L->dims);
   const int N = g.out_features(), K = g.in_features();
-  if (K % 8 != 0) return BQQ_ERR_UNSUPPORTED;   // 16-byte row pitch for the TMA descriptors
   if (!ws || ws_bytes < prefill_workspace_bytes(&L->dims, M)) return BQQ_ERR_WORKSPACE;
   if (((uintptr_t)ws & 255) != 0) return BQQ_ERR_MISALIGNED;
   uint8_t* wsb = reinterpret_cast<uint8_t*>(ws);
@@ -446,6 +363,13 @@ int prefill_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t
   uint16_t* xhi = reinterpret_cast<uint16_t*>(wsb + 256 + up256((size_t)2 * N * K * 2));
   uint16_t* xlo = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(xhi) + up256((size_t)M * K * 2));
   float* bound_parts = reinterpret_cast<float*>(wsb + 16);
+  if (M <= kFusedMaxM) {
+    const size_t cw = up256(fused_counter_words(g) * 4);
+    const int rc = fused_launch(L, x, x_dtype, M, ldx, y, y_dtype, ldy, reinterpret_cast<unsigned*>(wsb + 256), status, true,
+                                wsb + 256 + cw, nullptr, st);
+    if (rc != BQQ_ERR_UNSUPPORTED) return rc;
+  }
+  if (K % 8 != 0) return BQQ_ERR_UNSUPPORTED;   // 16-byte row pitch for the TMA descriptors
 
   if (cudaMemsetAsync(status, 0, 32, st) != cudaSuccess) return BQQ_ERR_CUDA;   // status word and bound parts
 

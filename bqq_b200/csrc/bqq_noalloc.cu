@@ -59,7 +59,7 @@ int bqq_forward_decode_noalloc(const BqqLayer* layer, const void* x, int x_dtype
   // every argument check comes before anything is enqueued: a rejected call leaves the stream untouched
   int rc = bqq_decode_check_args(layer, x, x_dtype, M, ldx, y, y_dtype, ldy, nullptr);
   if (rc) return rc;
-  const size_t need = decode_workspace_bytes(&layer->dims, M);
+  const size_t need = decode_min_workspace_bytes(&layer->dims, M);
   if (need == 0) return BQQ_ERR_UNSUPPORTED;
   if (need > kNoAllocBytes) return BQQ_ERR_SCRATCH_LIMIT;      // layer / batch too large for the fixed array
   void* scratch = nullptr;

@@ -159,4 +159,21 @@ __device__ __forceinline__ void rebuild_bit(RebuildAcc& r, const RebuildLane& L,
   }
 }
 
+// n bit layers in a row; words of bit layer b at y + b step and z + b step, its {a, b, c, .} at k[b kstep], to be multiplied
+// by f.  FIRST: they start the sums.
+template <int RT>
+__device__ __forceinline__ void rebuild_bits(RebuildAcc& r, const RebuildLane& L, const uint32_t* y, const uint32_t* z, int step,
+                                             const float4* k, int kstep, float f, int lane, int n, bool first) {
+  if (first) {
+    const float4 c = *k;
+    rebuild_bit<RT, true>(r, L, y, z, lane, c.x * f, c.y * f, c.z * f);
+    --n; y += step; z += step; k += kstep;
+  }
+#pragma unroll 1
+  for (; n > 0; --n, y += step, z += step, k += kstep) {
+    const float4 c = *k;
+    rebuild_bit<RT, false>(r, L, y, z, lane, c.x * f, c.y * f, c.z * f);
+  }
+}
+
 }  // namespace bqq

@@ -238,18 +238,9 @@ bqq_reconstruct_kernel(const ReconParams p) {
       const bool live = sub < h.patches;
       if (live) {
         const uint32_t* w = reinterpret_cast<const uint32_t*>(rsm + (size_t)((s * kReconGroups + grp) * nb) * kBitBytes) + sub;
-        int b = 0;
-        if (chunk == 0) {
-          const float4 k = st.coef[grp][0][sub];
-          d = k.w;
-          rebuild_bit<RT, true>(r, L, w, w + RT * 128, lane, k.x, k.y, k.z);
-          b = 1;
-        }
-#pragma unroll 1
-        for (; b < nbits; ++b) {
-          const float4 k = st.coef[grp][b][sub];
-          rebuild_bit<RT, false>(r, L, w + b * (kBitBytes / 4), w + b * (kBitBytes / 4) + RT * 128, lane, k.x, k.y, k.z);
-        }
+        const float4* k = &st.coef[grp][0][sub];
+        if (chunk == 0) d = k->w;
+        rebuild_bits<RT>(r, L, w, w + RT * 128, kBitBytes / 4, k, kGroup, 1.f, lane, nbits, chunk == 0);
       }
       const long long at = h.at + here;
       const int rows = h.rows, cols = h.cols;
@@ -264,36 +255,43 @@ bqq_reconstruct_kernel(const ReconParams p) {
       rebuild_end(r, d);
       WT* wp = reinterpret_cast<WT*>(p.W) + at;
       WT* lp = LO ? reinterpret_cast<WT*>(p.W_lo) + at : nullptr;
-      const bool whole = p.quads && rows == 32 && cols == 32;
-      auto row = [&](auto RR) {
-        constexpr int rr = decltype(RR)::value;
-        auto half = [&](int qh, float2 v01, float2 v23) {
-          WT* w = wp + 8 * rr * ldw + 16 * qh;
-          WT* lo = LO ? lp + 8 * rr * ldw + 16 * qh : nullptr;
-          if (whole) {
-            const WT2 w01 = WType<DT>::cvt2(v01.x, v01.y), w23 = WType<DT>::cvt2(v23.x, v23.y);
-            store_quad(w, w01, w23);
-            if (LO)
-              store_quad(lo, WType<DT>::cvt2(v01.x - WType<DT>::back(w01.x), v01.y - WType<DT>::back(w01.y)),
-                         WType<DT>::cvt2(v23.x - WType<DT>::back(w23.x), v23.y - WType<DT>::back(w23.y)));
-          } else if (g8 + 8 * rr < rows) {
-            const float v[4] = {v01.x, v01.y, v23.x, v23.y};
+      const bool quad0 = p.quads && 4 * t4 + 4 <= cols, quad1 = p.quads && 4 * t4 + 20 <= cols;
+      auto half = [&](auto RR, auto QH, bool quad, float2 v01, float2 v23) {
+        constexpr int rr = decltype(RR)::value, qh = decltype(QH)::value;
+        WT* w = wp + 8 * rr * ldw + 16 * qh;
+        WT* lo = LO ? lp + 8 * rr * ldw + 16 * qh : nullptr;
+        if (quad) {
+          const WT2 w01 = WType<DT>::cvt2(v01.x, v01.y), w23 = WType<DT>::cvt2(v23.x, v23.y);
+          store_quad(w, w01, w23);
+          if (LO)
+            store_quad(lo, WType<DT>::cvt2(v01.x - WType<DT>::back(w01.x), v01.y - WType<DT>::back(w01.y)),
+                       WType<DT>::cvt2(v23.x - WType<DT>::back(w23.x), v23.y - WType<DT>::back(w23.y)));
+        } else {
+          const float v[4] = {v01.x, v01.y, v23.x, v23.y};
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (4 * t4 + 16 * qh + e < cols) {
-                const WT t = WType<DT>::cvt(v[e]);
-                w[e] = t;
-                if (LO) lo[e] = WType<DT>::cvt(v[e] - WType<DT>::back(t));
-              }
-          }
-        };
-        half(0, rebuild_entry<rr, 0>(r), rebuild_entry<rr, 1>(r));
-        half(1, rebuild_entry<rr, 2>(r), rebuild_entry<rr, 3>(r));
+          for (int e = 0; e < 4; ++e)
+            if (4 * t4 + 16 * qh + e < cols) {
+              const WT t = WType<DT>::cvt(v[e]);
+              w[e] = t;
+              if (LO) lo[e] = WType<DT>::cvt(v[e] - WType<DT>::back(t));
+            }
+        }
       };
-      row(std::integral_constant<int, 0>());
-      row(std::integral_constant<int, 1>());
-      row(std::integral_constant<int, 2>());
-      row(std::integral_constant<int, 3>());
+      auto each_row = [&](auto WHOLE) {
+        auto row = [&](auto RR) {
+          constexpr int rr = decltype(RR)::value;
+          constexpr bool whole = decltype(WHOLE)::value;
+          if (!whole && g8 + 8 * rr >= rows) return;
+          half(RR, std::integral_constant<int, 0>(), whole || quad0, rebuild_entry<rr, 0>(r), rebuild_entry<rr, 1>(r));
+          half(RR, std::integral_constant<int, 1>(), whole || quad1, rebuild_entry<rr, 2>(r), rebuild_entry<rr, 3>(r));
+        };
+        row(std::integral_constant<int, 0>());
+        row(std::integral_constant<int, 1>());
+        row(std::integral_constant<int, 2>());
+        row(std::integral_constant<int, 3>());
+      };
+      if (p.quads && rows == 32 && cols == 32) each_row(std::true_type());
+      else each_row(std::false_type());
     }
     if (!ok && p.status && lane == 0) atomicExch(p.status, 1u);   // a bounded wait gave up: the entries are invalid
   }

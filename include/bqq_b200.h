@@ -159,7 +159,11 @@ int bqq_repack_u8_planes(const uint8_t* Y_packed, const uint8_t* Z_packed, const
  *   required.  Calls sharing a workspace
  *   must not overlap on the GPU.  Results do not depend on the number of row
  *   patches: a row shard reproduces its slice of the full output bit for bit.
- * bqq_forward_prefill: any M; rebuilds W once into the workspace and runs a
+ *   From 13 rows on (fewer for patch geometries that the kernel would pad badly)
+ *   W is instead rebuilt tile by tile in shared memory and multiplied by tcgen05 at
+ *   once, W as a pair of bf16 and x as it is or as a pair.
+ * bqq_forward_prefill: any M; up to 128 rows the same with W and x in fp16 (a pair
+ *   of bf16 each for fp32 x), else rebuilds W once into the workspace and runs a
  *   tcgen05 tensor-core GEMM (fp32 accumulate); replaces reconstruct_W_kernel +
  *   torch::mm (src/bqq_cuda.cu:198-246, 367-383).  The first word of the
  *   workspace is a status word: non-zero after the call completes means a
@@ -228,7 +232,8 @@ int bqq_prefill_status(const void* workspace, void* stream);
 /*
  * Number of kernels one bqq_forward_decode call enqueues for this layer shape and
  * M (1 or 2: short single-chunk layers at M = 1 prepare x inside the decode
- * kernel, all others launch a preparation kernel first); negative BQQ_ERR_* for
+ * kernel, and aligned bf16 rows of 32-column patches are multiplied as they are
+ * from 13 rows on; all others launch a preparation kernel first); negative BQQ_ERR_* for
  * bad arguments.  For launch accounting; the reference has no such query.
  */
 int bqq_decode_launches(const BqqDims* dims, int M);
@@ -368,7 +373,9 @@ int bqq_peer_status(const BqqPeerGroup* group, void* stream);
  * gather regions of all ranks while the rest of the kernel still runs, and a few
  * additional CTAs of the same grid wait (bounded) for the peers' row patches and
  * write the full rows [M, world*out_local] to `gathered`; the computing CTAs never
- * wait for them.  y_local [M, out_local] still receives this rank's columns.
+ * wait for them.  (Batches that bqq_forward_decode multiplies tile by tile are
+ * gathered by a kernel of its own behind it.)  y_local [M, out_local] still receives
+ * this rank's columns.
  * `fusion` (may be NULL) as in bqq_forward_decode_fused; a residual is this rank's
  * column slice [M, out_local] and is added before the outputs are sent.  Same
  * rules as bqq_forward_decode and bqq_peer_gather; 16-bit outputs need an even P.
