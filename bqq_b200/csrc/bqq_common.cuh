@@ -111,15 +111,32 @@ __device__ __forceinline__ float round_to(float v, int dt) {
 }
 
 // Power-of-two scale that maps a bound on |W| to at most 2^14 (fp16-safe range).
-// bound_parts = {max(|a|+|b|+|c|), max|d|}; |W| <= mult * parts[0] + parts[1], mult = bw * r.
-__device__ __forceinline__ float w_scale_from_bound(const float* bound_parts, float mult) {
-  const float bound = fmaf(mult, bound_parts[0], bound_parts[1]);
+__device__ __forceinline__ float scale_from_bound(float bound) {
   if (!(bound > 0.f) || !isfinite(bound)) return 1.f;
   int e;
   frexpf(bound, &e);                 // bound = f * 2^e, f in [0.5, 1)
   int s = 14 - e;
   s = max(-100, min(100, s));
   return exp2f((float)s);
+}
+// The same from the maxima that coef_bound_kernel left: [kBoundBlocks] of |a|+|b|+|c| and [kBoundBlocks] of |d|;
+// |W| <= mult * the first + the second, mult = bw * r.  All lanes of a warp call it.
+constexpr int kBoundBlocks = 256;
+__device__ __forceinline__ float w_scale_from_maxima(const float* maxima, float mult, int lane) {
+  float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+  for (int e = 0; e < kBoundBlocks / 128; ++e) {
+    const float4 u = reinterpret_cast<const float4*>(maxima)[e * 32 + lane];
+    const float4 v = reinterpret_cast<const float4*>(maxima + kBoundBlocks)[e * 32 + lane];
+    m0 = fmaxf(m0, fmaxf(fmaxf(u.x, u.y), fmaxf(u.z, u.w)));
+    m1 = fmaxf(m1, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+  return scale_from_bound(fmaf(mult, m0, m1));
 }
 
 // One slot of a peer gather region: (data word, sequence number) as ONE scalar 64-bit access at
@@ -178,7 +195,8 @@ size_t fused_workspace_bytes(const Geom& g, int M);    // 0: not for this many r
 size_t fused_counter_words(const Geom& g);
 int fused_launch(const BqqLayer* layer, const void* x, int x_dtype, int M, int64_t ldx, void* y, int y_dtype, int64_t ldy,
                  unsigned* counters, unsigned* status, bool clear, void* scratch, const BqqFusion* fusion, cudaStream_t stream);
-int coef_bound_launch(const BqqLayer* layer, float* bound_parts, cudaStream_t stream);   // bound_parts zero on entry
+// maxima of the coefficients, 2 x kBoundBlocks floats (NULL: none wanted); clears *status
+int coef_bound_launch(const BqqLayer* layer, float* maxima, unsigned* status, cudaStream_t stream);
 int prefill_launch(const BqqLayer* layer, const void* x, int x_dtype, int M, int64_t ldx, void* y,
                    int y_dtype, int64_t ldy, void* ws, size_t ws_bytes, cudaStream_t stream);
 size_t prefill_workspace_bytes(const BqqDims* dims, int M);

@@ -51,8 +51,7 @@ fused_prep_kernel(const XSource xs, int M, Geom g, int Kp, uint16_t* __restrict_
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 8; ++k) top = fmaxf(top, part[k]);
-    const float parts[2] = {0.f, top};
-    scale = w_scale_from_bound(parts, 0.f);
+    scale = scale_from_bound(top);
     if (threadIdx.x == 0 && blockIdx.x == 0) unscale[m] = 1.f / scale;
   }
   for (int k0 = (blockIdx.x * 256 + threadIdx.x) * 8; k0 < Kp; k0 += gridDim.x * 2048) {

@@ -327,8 +327,7 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
         }
 #pragma unroll
       for (int e = 16; e > 0; e >>= 1) bound = fmaxf(bound, __shfl_xor_sync(0xffffffffu, bound, e));
-      const float parts[2] = {0.f, bound};
-      const float s = w_scale_from_bound(parts, 0.f);
+      const float s = scale_from_bound(bound);
       if (lane == 0) {
         wscale[4 * set + quarter] = s;
         mbar_arrive(scaled + set);

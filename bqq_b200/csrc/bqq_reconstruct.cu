@@ -30,7 +30,7 @@ struct ReconParams {
   const void *a, *b, *c, *d;
   void* W;
   void* W_lo;                  // optional second part: W - round(W), same type and layout
-  const float* bound_parts;    // optional: entries are also scaled by w_scale_from_bound
+  const float* bound_parts;    // optional: entries are also scaled by w_scale_from_maxima
   float scale;
   int coef_dtype, w_dtype;
   int quads;                   // 1: four neighbouring entries of a row may be stored as one aligned word
@@ -193,7 +193,7 @@ bqq_reconstruct_kernel(const ReconParams p) {
     };
     coefficients();
     pdl_enter(p.pdl);
-    const float scale = p.bound_parts ? p.scale * w_scale_from_bound(p.bound_parts, (float)(g.bw * g.r)) : p.scale;
+    const float scale = p.bound_parts ? p.scale * w_scale_from_maxima(p.bound_parts, (float)(g.bw * g.r), lane) : p.scale;
     const float cscale = kind < 3 ? scale * kCoefScale : scale;
     for (int n = 0; n < nstages; ++n) {
       const int s = n % kReconStages;
@@ -354,38 +354,52 @@ int reconstruct_launch(const BqqLayer* L, void* W, void* W_lo, int w_dtype, floa
   return reconstruct_dispatch<2>(p, blocks, st);
 }
 
-// bound_parts[0] = max(|a|+|b|+|c|), bound_parts[1] = max|d| (both must be zero on entry: the caller clears them)
-__global__ void coef_bound_kernel(const void* a, const void* b, const void* c, const void* d, int dt, size_t nabc,
-                                  size_t nd, float* bound_parts) {
-  pdl_enter(kPdlWaitFirst);          // the bound words were cleared by a memset node: nothing to overlap with
+// maxima[block] = max(|a|+|b|+|c|), maxima[kBoundBlocks + block] = max|d| over the block's share of the coefficients
+// (maxima may be NULL); clears *status.  Every block writes its pair, so nothing has to be cleared before.
+__global__ void __launch_bounds__(256)
+coef_bound_kernel(const void* a, const void* b, const void* c, const void* d, int dt, size_t nabc, size_t nd, float* maxima,
+                  unsigned* status) {
+  pdl_enter(kPdlWaitFirst);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0u;
+  if (!maxima) return;
   float m0 = 0.f, m1 = 0.f;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nabc; t += (size_t)gridDim.x * blockDim.x)
+#pragma unroll 4
+  for (size_t t = blockIdx.x * 256 + threadIdx.x; t < nabc; t += kBoundBlocks * 256)
     m0 = fmaxf(m0, fabsf(load_as_float(a, t, dt)) + fabsf(load_as_float(b, t, dt)) + fabsf(load_as_float(c, t, dt)));
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nd; t += (size_t)gridDim.x * blockDim.x)
+#pragma unroll 4
+  for (size_t t = blockIdx.x * 256 + threadIdx.x; t < nd; t += kBoundBlocks * 256)
     m1 = fmaxf(m1, fabsf(load_as_float(d, t, dt)));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
     m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
   }
-  // one pair of atomics per block: the warps' maxima meet in shared memory first
   __shared__ float part[2][8];
   const int warp = threadIdx.x >> 5;
   if ((threadIdx.x & 31) == 0) { part[0][warp] = m0; part[1][warp] = m1; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) { m0 = fmaxf(m0, part[0][w]); m1 = fmaxf(m1, part[1][w]); }
-    // non-negative floats order like ints
-    atomicMax(reinterpret_cast<int*>(bound_parts), __float_as_int(m0));
-    atomicMax(reinterpret_cast<int*>(bound_parts) + 1, __float_as_int(m1));
+  if (threadIdx.x < 2) {
+    float m = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, part[threadIdx.x][w]);
+    maxima[threadIdx.x * kBoundBlocks + blockIdx.x] = m;
   }
 }
 
-int coef_bound_launch(const BqqLayer* L, float* bound_parts, cudaStream_t st) {
+int coef_bound_launch(const BqqLayer* L, float* maxima, unsigned* status, cudaStream_t st) {
   Geom g(L->dims);
   const size_t nabc = (size_t)g.bw * g.rw * g.cw, nd = (size_t)g.rw * g.cw;
-  int blocks = (int)((nabc + 255) / 256 < 296 ? (nabc + 255) / 256 : 296);
-  coef_bound_kernel<<<blocks, 256, 0, st>>>(L->a, L->b, L->c, L->d, L->coef_dtype, nabc, nd, bound_parts);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(maxima ? kBoundBlocks : 1);
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, coef_bound_kernel, L->a, L->b, L->c, L->d, (int)L->coef_dtype, nabc, nd, maxima,
+                         status) != cudaSuccess) { cudaGetLastError(); return BQQ_ERR_CUDA; }
   return launch_status();
 }
 

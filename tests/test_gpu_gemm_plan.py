@@ -1,0 +1,25 @@
+"""GPU: the prefill GEMM where its tile width, row halves and K split change: few tiles with a long K (the sums of a tile meet
+in a cluster), odd numbers of pieces per CTA, tile borders that cut row patches, every element type."""
+import pytest
+import torch
+
+from oracle import bqq_oracle as O
+from tests.helpers import oracle_forward_t, synth_layer
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize('rw,cw,M', [(2, 160, 129), (5, 64, 200), (12, 60, 333), (40, 90, 150), (9, 33, 700), (37, 40, 300),
+                                     (1, 96, 260)])
+def test_split_and_tile_rules(rw, cw, M):
+    from bqq_b200.bqq_modules import BinaryQuadratic, check_status
+    Y, Z, A, bias, X = synth_layer(2, rw, cw, 40, 32, 32, M, seed=rw + cw + M, bias=True)      # P = 40: borders cut row patches
+    bq = BinaryQuadratic(Y.float(), Z.float(), A, bias=bias).cuda()
+    for dt, tol in ((torch.float32, 1e-4), (torch.bfloat16, 1e-3 + 2 ** -8), (torch.float16, 1e-3 + 2 ** -10)):
+        Xd = X.to(dt)
+        with torch.no_grad():
+            y = bq(Xd.cuda())
+            again = bq(Xd.cuda())
+        assert torch.equal(y, again)                        # the exchange adds in a fixed order
+        assert O.max_rel_err(y.float().cpu().numpy(), oracle_forward_t(Y, Z, A, bias, Xd)) < tol
+    check_status()
