@@ -22,7 +22,7 @@
 // Every mbarrier wait is bounded by a clock budget; on expiry the kernel records
 // a status code in global memory, drains its copies and returns.
 //
-// The call is a chain of programmatic dependent launches over column panels of W (about one wave of
+// The call is a chain of programmatic dependent launches over column panels of W (one wave of
 // GEMM tiles each): bound, rebuild panel 0, stage x, then alternately multiply panel p and rebuild
 // panel p+1.  A GEMM waits for everything before it and then lets the next rebuild start at once, so the
 // rebuild of a panel (ALU work) runs beside the GEMM of the previous one (TMA and tensor pipe).
@@ -109,7 +109,7 @@ __device__ __forceinline__ void gemm_store(const GemmParams& p, const float (&f)
   }
 }
 
-template <int MT>
+template <int MT, bool PAIR>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
                 const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
@@ -117,7 +117,8 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
   constexpr uint32_t kAHalf = kBM * kBK * 2;              // one 128-row half of the A tile
   constexpr uint32_t kABytes = MT * kAHalf;
   const int BN = p.BN;
-  const uint32_t kBBytes = (uint32_t)BN * kBK * 2;
+  const int brows = PAIR ? BN / 2 : BN;                   // rows of the B tile that this CTA holds
+  const uint32_t kBBytes = (uint32_t)brows * kBK * 2;
   const uint32_t acc_cols = (uint32_t)BN;                 // tensor-memory columns of one accumulator
   uint32_t tmem_cols = 32;
   while (tmem_cols < acc_cols * MT) tmem_cols *= 2;
@@ -136,10 +137,14 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
   pdl_enter(kPdlWaitFirst);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int rank = (int)(blockIdx.x % (unsigned)p.split);
-  const int n0 = (int)(blockIdx.x / (unsigned)p.split + p.n_tile0) * BN;
+  const unsigned csize = (unsigned)p.split * (PAIR ? 2 : 1);
+  const int crank = (int)(blockIdx.x % csize);             // rank in the cluster: (share of K, half of a pair)
+  const int rank = PAIR ? crank >> 1 : crank, half = PAIR ? crank & 1 : 0;
+  const int n0 = (int)(blockIdx.x / csize + p.n_tile0) * BN;
   const int n_end = min(p.N, n0 + BN);
-  const int m0 = blockIdx.y * (kBM * MT);
+  // row half mt of this CTA starts at m0 + mt * mstep
+  constexpr int mstep = PAIR ? 2 * kBM : kBM;
+  const int m0 = blockIdx.y * (kBM * MT * (PAIR ? 2 : 1)) + half * kBM;
   const int kblocks = (p.K + kBK - 1) / kBK;
   const int all = kblocks * p.passes;
   const int it0 = (int)((long long)all * rank / p.split), it1 = (int)((long long)all * (rank + 1) / p.split);
@@ -152,11 +157,17 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
     mbar_init_fence();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();                  // the leader's barriers are initialised before the other half's copies report
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   bool ok = true;
@@ -168,23 +179,34 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
       int kb = it0 % kblocks, pass = it0 / kblocks;
       for (int it = 0; it < iters; ++it) {
         if (*failed || !mbar_wait(empty_bar + s, ph)) { *failed = 1; break; }
-        mbar_expect_tx(full_bar + s, kABytes + kBBytes);
         const CUtensorMap* ma = p.a_sel[pass] == 0 ? &map_a0 : &map_a1;
-        tma_load_2d(sA + s * kABytes, ma, full_bar + s, kb * kBK, m0);
-        tma_load_2d(sB + s * kBBytes, &map_b, full_bar + s, kb * kBK, p.b_row[pass] + n0);
+        if (PAIR) {
+          if (half == 0) mbar_expect_tx(full_bar + s, 2 * (kABytes + kBBytes));
+          const uint32_t bar = cluster_address(smem_u32(full_bar + s), (uint32_t)(crank & ~1));
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt)
+            tma_load_2d_pair(sA + s * kABytes + mt * kAHalf, ma, bar, kb * kBK, m0 + mt * mstep);
+          tma_load_2d_pair(sB + s * kBBytes, &map_b, bar, kb * kBK, p.b_row[pass] + n0 + half * brows);
+        } else {
+          mbar_expect_tx(full_bar + s, kABytes + kBBytes);
+          tma_load_2d(sA + s * kABytes, ma, full_bar + s, kb * kBK, m0);
+          tma_load_2d(sB + s * kBBytes, &map_b, full_bar + s, kb * kBK, p.b_row[pass] + n0);
+        }
         issued = it + 1;
         if (++kb == kblocks) { kb = 0; ++pass; }
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
-      if (*failed) {
-        // drain: copies already issued must land before the CTA exits
+      if (*failed && half == 0) {
+        // drain: copies already issued must land before the CTA exits (the leader's barriers count those of both halves,
+        // which leave together)
         int first = issued > p.stages ? issued - p.stages : 0;
         for (int it = first; it < issued; ++it)
           mbar_wait(full_bar + it % p.stages, (uint32_t)(it / p.stages) & 1u);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && half == 0) {
+      const uint16_t both = (uint16_t)(3u << (crank & ~1));
       int s = 0;
       uint32_t ph = 0;
       for (int it = 0; it < iters; ++it) {
@@ -195,13 +217,20 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
         for (int mt = 0; mt < MT; ++mt) {
           const uint64_t adesc = make_smem_desc(smem_u32(sA + s * kABytes + mt * kAHalf));
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)   // 16 elements = 32 bytes = 2 descriptor units per step
-            tc_mma_f16(tmem_base + (uint32_t)mt * acc_cols, adesc + 2 * k, bdesc + 2 * k, p.idesc, (it | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < kBK / 16; ++k) { // 16 elements = 32 bytes = 2 descriptor units per step
+            const uint32_t d = tmem_base + (uint32_t)mt * acc_cols, accum = (it | k) != 0 ? 1u : 0u;
+            if (PAIR) tc_mma_f16_pair(d, adesc + 2 * k, bdesc + 2 * k, p.idesc, accum);
+            else tc_mma_f16(d, adesc + 2 * k, bdesc + 2 * k, p.idesc, accum);
+          }
         }
-        tc_commit(empty_bar + s);            // frees the stage when these MMAs have read it
+        // frees the stage when these MMAs have read it
+        if (PAIR) tc_commit_pair(empty_bar + s, both);
+        else tc_commit(empty_bar + s);
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
-      tc_commit(acc_bar);                    // accumulator complete (or abandoned)
+      // accumulators complete (or abandoned)
+      if (PAIR) tc_commit_pair(acc_bar, both);
+      else tc_commit(acc_bar);
     }
   } else {
     ok = mbar_wait(acc_bar, 0) && !*failed;
@@ -223,7 +252,7 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
 #pragma unroll 1
       for (int q = 0; q < pieces; ++q) {
         const int mt = q / cpt, c = q - mt * cpt;
-        const int m = m0 + mt * kBM + quarter * 32 + lane;
+        const int m = m0 + mt * mstep + quarter * 32 + lane;
         uint32_t v[32];
         tc_ld32(mine + (uint32_t)mt * acc_cols + (uint32_t)(c * 32), v);
         tc_wait_ld();
@@ -259,7 +288,7 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
 #pragma unroll 1
       for (int q = rank; q < pieces; q += p.split) {
         const int mt = q / cpt, c = q - mt * cpt;
-        const int m = m0 + mt * kBM + quarter * 32 + lane;
+        const int m = m0 + mt * mstep + quarter * 32 + lane;
         if (m >= p.M || n0 + c * 32 >= n_end) continue;
         const uint8_t* src = sA + (size_t)(q / p.split) * p.split * kPiece + (quarter * 32 + lane) * 16;
         float o[32];
@@ -283,9 +312,11 @@ bqq_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constan
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
   }
   if (threadIdx.x == 0 && *failed) atomicExch(p.status, 1u);
+  if (PAIR) cluster_sync();                  // neither half leaves while the other may still signal it
 }
 
 // ---- x staging: any dtype / stride -> dense 16-bit rows (hi, lo for fp32) ----
@@ -404,20 +435,32 @@ size_t prefill_workspace_bytes(const BqqDims* dims, int M) {
 }
 
 struct GemmPlan {
-  int BN, MT, split, stages;
+  int BN, MT, split, pair, stages;
   size_t smem;
 };
 
+// Column panels: W is rebuilt and multiplied panel by panel, so that the rebuild of panel p + 1 runs beside the GEMM of panel
+// p.  Tiles of a panel along N: what fills the SMs once, but at most eight panels.
+static int panel_tiles(int tm, int tn) {
+  if ((long long)tm * tn <= 222) return tn;                       // one wave and a half: not worth another rebuild launch
+  const int tpp = std::max(std::max(1, 148 / tm), (tn + 7) / 8);
+  const int panels = (tn + tpp - 1) / tpp;
+  return (tn + panels - 1) / panels;
+}
+// CTA pairs (cta_group::2) load half of the B tile each.  That is worth the pairing where W does not fit the half of the L2 that
+// is near an SM: 8192 x 4096 at 2048 rows 168.9 -> 164.5 us, 4096^2 at 1000 rows of fp32 118 -> 111, smaller W no difference.
+constexpr size_t kPairBytes = 64u << 20;
 // Tile and K split with the smallest estimated time, in SM clocks.  A k-block of 64 costs a CTA the largest of its products
-// (3.9 clocks per column and row half, about half the tensor peak: the ring's waits and the power limit are in it), its
-// operands at 55 bytes per clock, and its share of the L2 (6200 bytes per clock for all SMs).  To that come the start of the
-// CTA, the stores of a 32-column piece and, for a K split, two cluster barriers and the exchange of the pieces.  Clusters do
-// not fill all 148 SMs (kSlots: what the occupancy query reports for this kernel).  Where a wave is not full the estimate
-// counts 0.6 of the empty part (small CTAs share an SM).  The constants were fitted to 22 shapes (384 to 28672 outputs, 140 to
-// 4096 rows, every tile and split timed): the choice is within 1 % of the best on average, 3 % at worst.
-// Measured, whole forward, against the power-of-two tiles without a split of before (us): 2048 x 2048, 3 bit layers, 333 rows
-// of fp32 57.6 -> 34; 1024 x 9632, 4 bit layers, 1422 rows of bf16 82.6 -> 61.
-static GemmPlan plan_gemm(int M, int N, int kblocks) {
+// (3.5 clocks per column and row half; the tensor peak would be 2, the waits of the ring and the power limit are in it), its
+// operands at 65 bytes per clock, and its share of the L2 (7300 bytes per clock for all SMs).  To that come the start of the
+// CTA, the stores of a 32-column piece, for a K split (one row half only) two cluster barriers and the exchange of the
+// pieces, and 43000 clocks per panel.  Clusters do not fill all 148 SMs (kSlots: what the occupancy query reports for this
+// kernel).  The constants were fitted to 32 shapes (288 to 28672 outputs, 140 to 4096 rows, every tile and split timed): the
+// choice is within 1 % of the best on average, 5 % at worst.
+// Measured, whole forward, against the power-of-two tiles without a split (us): 2048 x 2048, 3 bit layers, 333 rows of fp32
+// 57.6 -> 34; 1024 x 9632, 4 bit layers, 1422 rows of bf16 82.6 -> 61.  Panels of one wave each instead of at most four:
+// 14336 x 4096, 2048 rows 335 -> 240; 8192 x 4096, 2048 rows 181 -> 141.
+static GemmPlan plan_gemm(int M, int N, int kblocks, size_t w_bytes) {
   static const int kSlots[9] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
   GemmPlan best = {};
   double best_cost = 0;
@@ -425,42 +468,53 @@ static GemmPlan plan_gemm(int M, int N, int kblocks) {
     for (int BN = 32; BN <= 256; BN += 32) {
       const int tm = (M + kBM * MT - 1) / (kBM * MT), tn = (N + BN - 1) / BN;
       const size_t stage = (size_t)MT * kBM * kBK * 2 + (size_t)BN * kBK * 2;
-      const int stages = (int)std::min<size_t>(kMaxStages, (kGemmSmem - 2048) / stage);
       const int pieces = MT * BN / 32;
       for (int S = 1; S <= 8; ++S) {
         const size_t sums = S > 1 ? (size_t)((pieces + S - 1) / S) * S * 32 * kBM * 4 : 0;
-        if (sums + 2048 > (size_t)kGemmSmem || (S > 1 && kblocks / S < 4)) continue;
+        if (sums + 2048 > (size_t)kGemmSmem || (S > 1 && (MT > 1 || kblocks / S < 4))) continue;
         const double ctas = (double)tm * tn * S, slots = kSlots[S];
-        const double waves = 0.6 * std::ceil(ctas / slots) + 0.4 * std::max(1.0, ctas / slots);
-        const double block = std::max(3.9 * BN * MT, stage * std::max(1 / 55.0, std::min(ctas, slots) / 6200.0));
-        const double tail = 1700.0 + 460.0 * pieces + (S > 1 ? 730.0 + 950.0 * pieces : 0.0);
-        const double cost = waves * ((kblocks + S - 1) / S * block + tail);
+        const int tpp = S > 1 ? tn : panel_tiles(tm, tn);
+        const int panels = (tn + tpp - 1) / tpp;
+        const double waves = panels > 1 ? (double)panels * ((tpp * tm + 147) / 148) : std::ceil(ctas / slots);
+        const double busy = std::min(panels > 1 ? (double)tpp * tm : ctas, slots);
+        const double block = std::max(3.5 * BN * MT, stage * std::max(1 / 65.0, busy / 7300.0));
+        const double tail = 7000.0 + 470.0 * pieces + (S > 1 ? 1750.0 + 180.0 * pieces : 0.0);
+        const double cost = waves * ((kblocks + S - 1) / S * block + tail) + 43000.0 * panels;
         if (best.BN == 0 || cost < best_cost) {
           best_cost = cost;
-          best = {BN, MT, S, stages, 2048 + std::max((size_t)stages * stage, sums)};
+          best = {BN, MT, S, (S == 1 && tm % 2 == 0 && w_bytes >= kPairBytes) ? 1 : 0, 0, 0};
         }
       }
     }
+  const size_t stage = (size_t)best.MT * kBM * kBK * 2 + (size_t)best.BN / (best.pair ? 2 : 1) * kBK * 2;
+  const int pieces = best.MT * best.BN / 32;
+  best.stages = (int)std::min<size_t>(kMaxStages, (kGemmSmem - 2048) / stage);
+  const size_t sums = best.split > 1 ? (size_t)((pieces + best.split - 1) / best.split) * best.split * 32 * kBM * 4 : 0;
+  best.smem = 2048 + std::max((size_t)best.stages * stage, sums);
+  // a CTA of a pair is alone on its SM: two pairs that wait for each other's tensor memory cannot meet
+  if (best.pair) best.smem = std::max(best.smem, (size_t)116 * 1024);
   return best;
 }
 
 // tiles [tile0, tile0 + ntiles) along N, all of M
 static int launch_gemm(const GemmPlan& pl, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& b, GemmParams p,
                        int tile0, int ntiles, cudaStream_t st) {
-  auto kern = pl.MT == 2 ? bqq_gemm_kernel<2> : bqq_gemm_kernel<1>;
+  auto kern = pl.pair ? (pl.MT == 2 ? bqq_gemm_kernel<2, true> : bqq_gemm_kernel<1, true>)
+                      : (pl.MT == 2 ? bqq_gemm_kernel<2, false> : bqq_gemm_kernel<1, false>);
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem) != cudaSuccess) return BQQ_ERR_CUDA;
   p.n_tile0 = tile0;
   cudaLaunchAttribute attr[2] = {pdl_attribute()};
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)pl.split;
+  const int cluster = pl.split * (pl.pair ? 2 : 1), rows = kBM * pl.MT * (pl.pair ? 2 : 1);
+  attr[1].val.clusterDim.x = (unsigned)cluster;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ntiles * pl.split, (p.M + kBM * pl.MT - 1) / (kBM * pl.MT));
+  cfg.gridDim = dim3(ntiles * cluster, (p.M + rows - 1) / rows);
   cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = pl.smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = pl.split > 1 ? 2 : 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, kern, a0, a1, b, p) != cudaSuccess) { cudaGetLastError(); return BQQ_ERR_CUDA; }
   return launch_status();
 }
@@ -487,16 +541,12 @@ int prefill_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t
 
   const bool f16 = x_dtype != BQQ_F32;
   const bool split_x = x_dtype == BQQ_F32;
-  const GemmPlan pl = plan_gemm(M, N, (K + kBK - 1) / kBK * (split_x ? 3 : 1));
-  const int BN = pl.BN, MT = pl.MT;
-  // Column panels of W of about one wave of GEMM tiles each (at most 4): the rebuild of panel p+1 runs beside the
-  // GEMM of panel p.  A row patch that a panel border cuts is rebuilt with the first of the two.
-  const int tiles_n = (N + BN - 1) / BN, tiles_m = (M + kBM * MT - 1) / (kBM * MT);
-  int panels = pl.split > 1 ? 1 : (int)(((long long)tiles_n * tiles_m + 74) / 148);
-  panels = panels < 1 ? 1 : (panels > 4 ? 4 : panels);
-  if (panels > tiles_n) panels = tiles_n;
-  const int tiles_pp = (tiles_n + panels - 1) / panels;
-  panels = (tiles_n + tiles_pp - 1) / tiles_pp;
+  const GemmPlan pl = plan_gemm(M, N, (K + kBK - 1) / kBK * (split_x ? 3 : 1), (size_t)N * K * (split_x ? 4 : 2));
+  const int BN = pl.BN;
+  // a row patch that a panel border cuts is rebuilt with the first of the two panels
+  const int tiles_n = (N + BN - 1) / BN, tiles_m = (M + kBM * pl.MT - 1) / (kBM * pl.MT);
+  const int tiles_pp = pl.split > 1 ? tiles_n : panel_tiles(tiles_m, tiles_n);
+  const int panels = (tiles_n + tiles_pp - 1) / tiles_pp;
   auto panel_rows = [&](int pnl, int* i0, int* i1) {           // row patches of panel pnl
     const int c0 = pnl * tiles_pp * BN, c1 = std::min(N, (pnl + 1) * tiles_pp * BN);
     *i0 = (c0 + g.P - 1) / g.P;
@@ -510,13 +560,14 @@ int prefill_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t
   float* unscale = reinterpret_cast<float*>(xlo);            // the lo region is free when x has 16 bits
   const float* row_unscale = x_dtype == BQQ_BF16 ? unscale : nullptr;
 
+  const uint32_t abox = pl.pair ? kBM : kBM * pl.MT;
   CUtensorMap ma0, ma1, mb;
-  int rc = make_map(&ma0, a_ptr, !f16, (uint64_t)M, (uint64_t)K, (uint64_t)a_ld, kBM * MT);
+  int rc = make_map(&ma0, a_ptr, !f16, (uint64_t)M, (uint64_t)K, (uint64_t)a_ld, abox);
   if (rc) return rc;
   rc = make_map(&ma1, split_x ? (const void*)xlo : a_ptr, !f16, (uint64_t)M, (uint64_t)K,
-                split_x ? (uint64_t)K : (uint64_t)a_ld, kBM * MT);
+                split_x ? (uint64_t)K : (uint64_t)a_ld, abox);
   if (rc) return rc;
-  rc = make_map(&mb, W, !f16, (uint64_t)(f16 ? N : 2 * N), (uint64_t)K, (uint64_t)K, (uint32_t)BN);
+  rc = make_map(&mb, W, !f16, (uint64_t)(f16 ? N : 2 * N), (uint64_t)K, (uint64_t)K, (uint32_t)(pl.pair ? BN / 2 : BN));
   if (rc) return rc;
 
   GemmParams p;
@@ -535,7 +586,7 @@ int prefill_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t
   }
   // instruction descriptor: fp32 accumulate, A and B in the same 16-bit format, both K-major
   const uint32_t fmt = f16 ? 0u : 1u;
-  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((pl.pair ? 2 * kBM : kBM) >> 4) << 24);
 
   // 1. (16-bit x) bound on |W| for the power-of-two scale of the fp16 weight.  fp16 and bf16 activations use one
   //    fp16 W (bf16 rows are re-staged as scaled fp16, exact); fp32 activations use the bf16 hi + lo pair.

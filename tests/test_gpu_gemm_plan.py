@@ -23,3 +23,18 @@ def test_split_and_tile_rules(rw, cw, M):
         assert torch.equal(y, again)                        # the exchange adds in a fixed order
         assert O.max_rel_err(y.float().cpu().numpy(), oracle_forward_t(Y, Z, A, bias, Xd)) < tol
     check_status()
+
+
+@pytest.mark.parametrize('rw,cw,M,dtype', [(1100, 32, 300, torch.bfloat16), (900, 40, 2100, torch.float16), (520, 64, 256, torch.float32)])
+def test_pairs_and_panels(rw, cw, M, dtype):
+    """W of more than 64 MB: column panels of one wave each, and CTA pairs where the row tiles are even."""
+    from bqq_b200.bqq_modules import BinaryQuadratic, check_status
+    Y, Z, A, _, X = synth_layer(1, rw, cw, 32, 32, 8, M, seed=rw, x_dtype=dtype)
+    bq = BinaryQuadratic(Y.float(), Z.float(), A).cuda()
+    with torch.no_grad():
+        y = bq(X.cuda()).float()
+        W = bq.get_weight(torch.float32)
+        ref = X.cuda().double() @ W.double().T
+    tol = 1e-4 if dtype == torch.float32 else 1e-3 + (2 ** -8 if dtype == torch.bfloat16 else 2 ** -10)
+    assert ((y - ref).abs().max() / ref.abs().max()).item() < tol
+    check_status()
