@@ -151,7 +151,7 @@ int decode_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t 
   p.x_dtype = x_dtype; p.y_dtype = y_dtype; p.bias_dtype = L->bias_dtype;
   p.M = M; p.bw = g.bw; p.rw = g.rw; p.cw = g.cw; p.P = g.P; p.Q = g.Q;
   p.PTg = g.PT; p.QTg = g.QT; p.RTg = g.RT; p.JG = g.JG; p.NS = g.NS;
-  p.sgw = pl.sgw; p.bpc = pl.bpc; p.nchunks = pl.nchunks; p.mtiles = pl.mtiles;
+  p.sgw = pl.sgw; p.bpc = pl.bpc; p.nbg = g.bw / pl.bpc; p.nchunks = pl.nchunks; p.mtiles = pl.mtiles;
   char* wsb = reinterpret_cast<char*>(ws);
   p.counters = reinterpret_cast<unsigned*>(wsb);
   p.xdig = reinterpret_cast<const uint8_t*>(wsb + kCounterBytes);

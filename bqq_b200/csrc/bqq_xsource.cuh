@@ -71,15 +71,51 @@ __device__ __forceinline__ void load_x_quad(const XSource& s, int m, int n0, flo
     for (int e = 0; e < 4; ++e) v[e] = v[e] / (1.f + __expf(-v[e])) * u[e];
   }
 }
+// Four consecutive elements as they lie in memory (aligned to four elements), and as floats: several loads can be under way
+// before the first is converted.
+__device__ __forceinline__ uint4 load_raw4(const void* base, size_t idx, bool f32) {
+  if (f32) return *reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(base) + idx);
+  const uint2 q = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(base) + idx);
+  return make_uint4(q.x, q.y, 0u, 0u);
+}
+__device__ __forceinline__ void raw4_to_float(const uint4& r, int dt, float (&v)[4]) {
+  if (dt == BQQ_F32) {
+    v[0] = __uint_as_float(r.x); v[1] = __uint_as_float(r.y); v[2] = __uint_as_float(r.z); v[3] = __uint_as_float(r.w);
+  } else if (dt == BQQ_BF16) {
+    v[0] = __uint_as_float(r.x << 16); v[1] = __uint_as_float(r.x & 0xFFFF0000u);
+    v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xFFFF0000u);
+  } else {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
+}
+// whether quads at multiples of four elements behind element `idx` can be read with load_raw4
+__device__ __forceinline__ bool raw4_aligned(const void* base, size_t idx, int dt) {
+  return dt == BQQ_F32 ? ((reinterpret_cast<uintptr_t>(base) + 4 * idx) & 15) == 0
+                       : ((reinterpret_cast<uintptr_t>(base) + 2 * idx) & 7) == 0;
+}
 // Sum of squares of row m over this thread's share of the columns (threads tid, tid + n, ...).
 __device__ __forceinline__ float row_sumsq_share(const XSource& s, int m, int tid, int nthreads) {
   float acc = 0.f;
-  if ((s.n_in & 3) == 0) {
-    for (int n = 4 * tid; n < s.n_in; n += 4 * nthreads) {
-      float v[4];
-      load_quad(s.x, (size_t)m * s.ld + n, s.dtype, v);
-      acc = fmaf(v[0], v[0], acc); acc = fmaf(v[1], v[1], acc);
-      acc = fmaf(v[2], v[2], acc); acc = fmaf(v[3], v[3], acc);
+  if ((s.n_in & 3) == 0 && raw4_aligned(s.x, (size_t)m * s.ld, s.dtype)) {
+    // eight quads in flight: one round trip for 4096 columns and 128 threads
+    constexpr int kAhead = 8;
+    for (int n0 = 4 * tid; n0 < s.n_in; n0 += 4 * kAhead * nthreads) {
+      uint4 r[kAhead];
+      const bool f32 = s.dtype == BQQ_F32;
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const int n = n0 + 4 * k * nthreads;
+        r[k] = n < s.n_in ? load_raw4(s.x, (size_t)m * s.ld + n, f32) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        float v[4];
+        raw4_to_float(r[k], s.dtype, v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc = fmaf(v[e], v[e], acc);
+      }
     }
   } else {
     for (int n = tid; n < s.n_in; n += nthreads) {
