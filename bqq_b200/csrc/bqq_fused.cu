@@ -96,7 +96,7 @@ namespace {
 
 struct FusedPlan {
   bool ok;
-  int N, nb, ns, nx, nw, tiles, chunks, chunk_stages, stages, Kp;
+  int N, nb, ns, nx, tiles, chunks, chunk_stages, stages, Kp;
   size_t smem, partial_bytes, x_bytes;
 };
 
@@ -109,23 +109,19 @@ FusedPlan make_plan(const Geom& g, int M, int NP, bool any_rows) {
   if (pl.N > (NP == 3 ? 64 : kFusedMaxN)) return pl;
   const int RT = g.RT;
   // Shared memory: at least two of everything, with as many bit layers per plane stage as that leaves room for; then deeper
-  // rings while there is room.  x first (a round trip for x is longer than a stage), then W buffers (they let the
-  // rebuild run ahead while x is being prepared), then planes.
+  // rings while there is room, x first (a round trip for x is longer than a stage).
   pl.nb = 0;
-  auto fits = [&](int nb, int ns, int nx, int nw) { return (size_t)FusedSmem(NP, RT, pl.N, nb, ns, nx, nw).total <= kMaxSmem; };
+  auto fits = [&](int nb, int ns, int nx) { return (size_t)FusedSmem(NP, RT, pl.N, nb, ns, nx).total <= kMaxSmem; };
   for (int nb = std::min(g.bw, kFusedBits / RT); nb >= 1 && !pl.nb; --nb) {
-    if (!fits(nb, 2, 2, 2)) continue;
+    if (!fits(nb, 2, 2)) continue;
     pl.nb = nb;
-    pl.ns = pl.nx = pl.nw = 2;
+    pl.ns = pl.nx = 2;
     for (bool more = true; more;) {
       more = false;
-      if (pl.nx < 3 && fits(nb, pl.ns, pl.nx + 1, pl.nw)) { ++pl.nx; more = true; }
-      if (pl.ns < 3 && fits(nb, pl.ns + 1, pl.nx, pl.nw)) { ++pl.ns; more = true; }
-      if (pl.nw < 4 && fits(nb, pl.ns, pl.nx, pl.nw + 1)) { ++pl.nw; more = true; }
-      if (!more && pl.nx < 4 && fits(nb, pl.ns, pl.nx + 1, pl.nw)) { ++pl.nx; more = true; }
-      if (!more && pl.ns < kFusedMaxPlaneStages && fits(nb, pl.ns + 1, pl.nx, pl.nw)) { ++pl.ns; more = true; }
+      if (pl.nx < 4 && fits(nb, pl.ns, pl.nx + 1)) { ++pl.nx; more = true; }
+      if (pl.ns < kFusedMaxPlaneStages && fits(nb, pl.ns + 1, pl.nx)) { ++pl.ns; more = true; }
     }
-    pl.smem = FusedSmem(NP, RT, pl.N, nb, pl.ns, pl.nx, pl.nw).total;
+    pl.smem = FusedSmem(NP, RT, pl.N, nb, pl.ns, pl.nx).total;
   }
   if (!pl.nb) return pl;
   pl.stages = g.JG * g.QT;
@@ -207,7 +203,7 @@ int fused_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t l
   p.coef_dtype = L->coef_dtype; p.bias_dtype = L->bias_dtype;
   p.g = g;
   p.M = M; p.N = pl.N;
-  p.nb = pl.nb; p.ns = pl.ns; p.nx = pl.nx; p.nw = pl.nw;
+  p.nb = pl.nb; p.ns = pl.ns; p.nx = pl.nx;
   p.row_unscale = NP == 1 && x_dtype == BQQ_BF16 ? unscale : nullptr;
   p.tiles = pl.tiles; p.chunks = pl.chunks; p.chunk_stages = pl.chunk_stages; p.stages = pl.stages;
   // fp32 accumulators, both operands fp16 or bf16, K-major; M = 128, N rows of x

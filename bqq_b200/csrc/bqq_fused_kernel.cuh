@@ -1,4 +1,4 @@
-// Forward for a few rows up to a few dozen: the dense weight exists only as tiles in shared memory.
+// Forward for a few rows up to a few dozen: the dense weight exists only as tiles in tensor memory.
 //   y[m, o] = sum_k W[o, k] x[m, k],  W rebuilt from the planes tile by tile and multiplied by tcgen05 at once.
 // Replaces the M > 1 branch of bqq_forward (neural_network_compression/src/bqq_cuda.cu:327-383) for these batches.
 //
@@ -12,8 +12,10 @@
 // which is the order of x itself for patches of 32 columns; other patches have x staged in that order, zeros in the
 // padding.  CTA = 16 compute warps (row block x col patch: one 32x32 block of W per stage each) and four
 // helpers: plane words by TMA ([Y of all row blocks | Z of all] [bit] in a stage), coefficients as floats, x by TMA,
-// tcgen05 issue.  Two W buffers in the
-// 128-byte-swizzled K-major layout; accumulators D[128 rows of W][N rows of x] in tensor memory, two sets.
+// tcgen05 issue.  W is operand A and lives in tensor memory (lane = row, two neighbouring k per column): the registers of a
+// finished 32x32 block are what two 16x256b stores take, against sixteen 4-byte stores into swizzled shared memory, a
+// proxy fence and up to 128 KB of buffers before.  Three or four W buffers, two sets of accumulators D[128 rows of W][N
+// rows of x] beside them.
 // Formats, accumulated in fp32 (NP products per tile):
 //   1  W in fp16, x in fp16: 16-bit x of more than 16 rows.  Every block of 32 rows of an item is scaled by a power of two
 //      (the bound on its entries maps to 2^14), bf16 rows of x are too; both are taken out of the sums.
@@ -23,9 +25,9 @@
 // in order by the CTA that finishes a tile last, so a row shard gives the same bits as the whole layer.  CTAs walk the
 // items; the sums of an item leave tensor memory while the next item is already being rebuilt, and the chunks are added up
 // at the end.
-// Measured (us, before -> with this kernel): 8192 x 28672, 3 bit layers of rank 64, 32 rows 461 (rebuild into memory and
-// GEMM) -> 375; 4096 x 4096, 2 bit layers, 64 rows 43.3 -> 28.2; 4096 x 14336, 3 bit layers, 16 rows 104.7 (decode kernel) ->
-// 75.6; P = 96, Q = 40, r = 33, 5 rows 25.0 -> 19.5.
+// Measured (us, before -> with this kernel, W in shared memory -> in tensor memory): 8192 x 28672, 3 bit layers of rank 64,
+// 32 rows 461 (rebuild into memory and GEMM) -> 375 -> 327; 4096 x 4096, 2 bit layers, 64 rows 43.3 -> 27.3 -> 26.0;
+// 4096 x 14336, 3 bit layers, 16 rows 104.7 (decode kernel) -> 75.8 -> 66.4; P = 96, Q = 40, r = 33, 5 rows 25.0 -> 19.2.
 #pragma once
 #include "bqq_rebuild.cuh"
 #include "bqq_tc.cuh"
@@ -58,7 +60,7 @@ struct FusedParams {
   int coef_dtype, bias_dtype, y_dtype, res_dtype;
   Geom g;
   int M, N;
-  int nb, ns, nx, nw;          // bit layers per plane stage; plane stages; x stages; W buffers
+  int nb, ns, nx;              // bit layers per plane stage; plane stages; x stages
   const float* row_unscale;    // NP = 1: factor of every row of x, or NULL
   int joint;                   // 1: one copy brings the planes of the tile's four row patches (PT = 1, all bit layers)
   int tiles, chunks, chunk_stages, stages;   // stages = JG * QT in all
@@ -67,18 +69,15 @@ struct FusedParams {
 
 // Shared-memory layout in bytes, host and device.
 struct FusedSmem {
-  int w, x, planes, coef, total;
-  int w_part, w_buf, x_part, x_stage, plane_group, plane_stage, coef_stage;
-  __host__ __device__ FusedSmem(int NP, int RT, int N, int nb, int ns, int nx, int nw) {
-    w_part = kFusedTile * kFusedStageCols * 2;                 // hi or lo: two 128 x 64 tiles
-    w_buf = (NP == 1 ? 1 : 2) * w_part;
+  int x, planes, coef, total;
+  int x_part, x_stage, plane_group, plane_stage, coef_stage;
+  __host__ __device__ FusedSmem(int NP, int RT, int N, int nb, int ns, int nx) {
     x_part = N * kFusedStageCols * 2;
     x_stage = x_part * (NP == 3 ? 2 : 1);
     plane_group = nb * RT * 1024;
     plane_stage = 4 * plane_group;
     coef_stage = 4 * nb * kGroup * 16;
     int o = 1024;                                              // barriers and flags (the base is rounded up to 1024)
-    w = o; o += nw * w_buf;
     x = o; o += nx * x_stage;
     planes = o; o += ns * plane_stage;
     coef = o; o += ns * coef_stage;
@@ -158,7 +157,7 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
                  const __grid_constant__ CUtensorMap map_y, const __grid_constant__ CUtensorMap map_z, const FusedParams p) {
   extern __shared__ __align__(1024) uint8_t fsm[];
   uint8_t* base = fsm + ((1024u - (smem_u32(fsm) & 1023u)) & 1023u);   // (pointer arithmetic: stays a shared address)
-  const FusedSmem L(NP, RT, p.N, p.nb, p.ns, p.nx, p.nw);
+  const FusedSmem L(NP, RT, p.N, p.nb, p.ns, p.nx);
   uint64_t* full = reinterpret_cast<uint64_t*>(base);                   // planes and coefficients of a stage are there
   uint64_t* used = full + kFusedMaxPlaneStages;
   uint64_t* xfull = used + kFusedMaxPlaneStages;                        // x of a stage
@@ -181,12 +180,16 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
   const int items = p.tiles * p.chunks;
   const int nchunks = (g.bw + p.nb - 1) / p.nb;                         // plane stages of a block
   const uint32_t acc_cols = (uint32_t)(p.N <= 16 ? 16 : p.N <= 32 ? 32 : p.N <= 64 ? 64 : 128);
-  const uint32_t tmem_cols = 2 * acc_cols;
+  constexpr uint32_t kWPart = kFusedStageCols / 2;                      // tensor-memory columns of a W buffer: hi, then lo
+  constexpr uint32_t kWCols = NP == 1 ? kWPart : 2 * kWPart;
+  constexpr int kWBufs = NP == 1 ? 4 : 3;
+  constexpr uint32_t tmem_cols = 512;
+  static_assert((NP == 1 ? 256 : NP == 2 ? 128 : 128) + kWBufs * kWCols <= tmem_cols, "");
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.ns; ++s) { mbar_init(full + s, 1 + 32); mbar_init(used + s, kFusedWarps); }
     for (int s = 0; s < p.nx; ++s) { mbar_init(xfull + s, 1); mbar_init(xfree + s, 1); }
-    for (int s = 0; s < p.nw; ++s) { mbar_init(wfull + s, kFusedWarps); mbar_init(wfree + s, 1); }
+    for (int s = 0; s < kWBufs; ++s) { mbar_init(wfull + s, kFusedWarps); mbar_init(wfree + s, 1); }
     for (int s = 0; s < 2; ++s) {
       mbar_init(scaled + s, 4);
       mbar_init(accfull + s, 1);
@@ -206,6 +209,7 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   auto wait = [&](uint64_t* bar, uint32_t phase) {                      // bounded; once one gave up, none waits any more
+    if (mbar_try_wait(bar, phase)) return true;
     if (*failed) return false;
     if (mbar_wait(bar, phase)) return true;
     *failed = 1;
@@ -220,15 +224,9 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
   if (warp < kFusedWarps) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFusedComputeRegs));
     // ---- rebuild ---------------------------------------------------------------------------------------
-    const int rb = warp >> 2, sub = warp & 3;
-    const int g8 = lane >> 2, t4 = lane & 3;
-    const RebuildLane RL = rebuild_lane<true>(lane);
-    // where this lane's entries go: row 32 rb + g8 (+ 8 rr: 1024 bytes), 64-column tile sub / 2, 16-byte piece
-    // 4 (sub & 1) + 2 qh + (t >> 1) of the row, swizzled by the row, pair x ^ (t >> 1) of the piece's half
-    const uint32_t wrow = smem_u32(base + L.w) + (sub >> 1) * (L.w_part / 2) + (32 * rb + g8) * 128 + 8 * (t4 & 1);
-    const uint32_t piece = 4 * (sub & 1) + (t4 >> 1);
-    const uint32_t at0 = wrow + ((piece ^ g8) << 4), at1 = wrow + (((piece + 2) ^ g8) << 4);
-    const uint32_t x0 = 4 * (t4 >> 1), x1 = 4 - x0;                    // byte offset of pair x = 0 and x = 1
+    const int rb = warp & 3, sub = warp >> 2;                          // a warp reaches the tensor-memory lanes 32 (warp % 4) ...
+    const RebuildLane RL = rebuild_lane(lane);
+    const uint32_t wt = tmem + 2 * acc_cols + 16 * sub + ((uint32_t)(32 * rb) << 16);
     RebuildAcc r;
     float d = 0.f;
     RingPos ps, ws;
@@ -259,40 +257,47 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
           if (lane == 0) mbar_arrive(used + ps.slot);
           ps.next(p.ns);
         }
-        if (wn >= p.nw) wait(wfree + ws.slot, ws.phase ^ 1u);
+        if (wn >= kWBufs) wait(wfree + ws.slot, ws.phase ^ 1u);
+        __syncwarp();
+        tc_fence_after();
         if (there) {
           rebuild_end(r, d * f);
-          const uint32_t hi = (uint32_t)(ws.slot * L.w_buf);
-          const uint32_t lo = hi + (uint32_t)L.w_part;
-          auto put = [&](auto RR, uint32_t at, float2 v, uint32_t xo) {
-            constexpr int rr = decltype(RR)::value;
-            if (NP == 1) {
-              const __half2 h = __floats2half2_rn(v.x, v.y);
-              store_shared_u32(at + hi + rr * 1024 + xo, *reinterpret_cast<const uint32_t*>(&h));
-              return;
-            }
-            const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
-            const uint32_t hw = *reinterpret_cast<const uint32_t*>(&h);
-            store_shared_u32(at + hi + rr * 1024 + xo, hw);
-            const __nv_bfloat162 l = __floats2bfloat162_rn(v.x - __uint_as_float(hw << 16), v.y - __uint_as_float(hw & 0xFFFF0000u));
-            store_shared_u32(at + lo + rr * 1024 + xo, *reinterpret_cast<const uint32_t*>(&l));
+          // entry pairs of rows g + 8 rr: 32-bit columns 8 qh + 2 t + x of the lane's quarter, which is their order in K
+          auto rows16 = [&](auto MT) {
+            constexpr int mt = decltype(MT)::value;
+            uint32_t hi[8], lo[8];
+            auto put = [&](auto K, float2 v) {
+              constexpr int k = decltype(K)::value;
+              if (NP == 1) {
+                const __half2 h = __floats2half2_rn(v.x, v.y);
+                hi[k] = *reinterpret_cast<const uint32_t*>(&h);
+                return;
+              }
+              const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+              hi[k] = *reinterpret_cast<const uint32_t*>(&h);
+              const __nv_bfloat162 l = __floats2bfloat162_rn(v.x - __uint_as_float(hi[k] << 16), v.y - __uint_as_float(hi[k] & 0xFFFF0000u));
+              lo[k] = *reinterpret_cast<const uint32_t*>(&l);
+            };
+            put(std::integral_constant<int, 0>(), rebuild_entry<2 * mt, 0>(r));
+            put(std::integral_constant<int, 1>(), rebuild_entry<2 * mt, 1>(r));
+            put(std::integral_constant<int, 2>(), rebuild_entry<2 * mt + 1, 0>(r));
+            put(std::integral_constant<int, 3>(), rebuild_entry<2 * mt + 1, 1>(r));
+            put(std::integral_constant<int, 4>(), rebuild_entry<2 * mt, 2>(r));
+            put(std::integral_constant<int, 5>(), rebuild_entry<2 * mt, 3>(r));
+            put(std::integral_constant<int, 6>(), rebuild_entry<2 * mt + 1, 2>(r));
+            put(std::integral_constant<int, 7>(), rebuild_entry<2 * mt + 1, 3>(r));
+            const uint32_t at = wt + ws.slot * kWCols + ((uint32_t)(16 * mt) << 16);
+            tc_st_16x256b_x2(at, hi);
+            if (NP != 1) tc_st_16x256b_x2(at + kWPart, lo);
           };
-          auto row = [&](auto RR) {
-            constexpr int rr = decltype(RR)::value;
-            put(RR, at0, rebuild_entry<rr, 0>(r), x0);
-            put(RR, at0, rebuild_entry<rr, 1>(r), x1);
-            put(RR, at1, rebuild_entry<rr, 2>(r), x0);
-            put(RR, at1, rebuild_entry<rr, 3>(r), x1);
-          };
-          row(std::integral_constant<int, 0>());
-          row(std::integral_constant<int, 1>());
-          row(std::integral_constant<int, 2>());
-          row(std::integral_constant<int, 3>());
+          rows16(std::integral_constant<int, 0>());
+          rows16(std::integral_constant<int, 1>());
+          tc_wait_st();
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before the tensor core reads it
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(wfull + ws.slot);
-        ws.next(p.nw);
+        ws.next(kWBufs);
         ++wn;
       }
     }
@@ -535,28 +540,28 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
         for (int t = t0; t < t1; ++t) {
           if (!wait(xfull + xs.slot, xs.phase) || !wait(wfull + ws.slot, ws.phase)) break;
           tc_fence_after();
-          const uint32_t w0 = smem_u32(base + L.w + ws.slot * L.w_buf), xa = smem_u32(base + L.x + xs.slot * L.x_stage);
+          const uint32_t wa = tmem + 2 * acc_cols + ws.slot * kWCols, xa = smem_u32(base + L.x + xs.slot * L.x_stage);
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            const uint64_t whi = make_smem_desc(w0 + k * (L.w_part / 2)), wlo = make_smem_desc(w0 + L.w_part + k * (L.w_part / 2));
+            const uint32_t whi = wa + 32 * k, wlo = whi + kWPart;
             const uint64_t xhi = make_smem_desc(xa + k * (L.x_part / 2));
 #pragma unroll
-            for (int e = 0; e < 4; ++e)                // 16 elements = 32 bytes = 2 descriptor units per step
-              tc_mma_f16(dtm, whi + 2 * e, xhi + 2 * e, p.idesc, (t != t0 || (k | e) != 0) ? 1u : 0u);
+            for (int e = 0; e < 4; ++e)                // 16 elements = 32 bytes: 8 columns of W, 2 descriptor units of x
+              tc_mma_f16_ts(dtm, whi + 8 * e, xhi + 2 * e, p.idesc, (t != t0 || (k | e) != 0) ? 1u : 0u);
             if (NP >= 2) {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) tc_mma_f16(dtm, wlo + 2 * e, xhi + 2 * e, p.idesc, 1u);
+              for (int e = 0; e < 4; ++e) tc_mma_f16_ts(dtm, wlo + 8 * e, xhi + 2 * e, p.idesc, 1u);
             }
             if (NP == 3) {
               const uint64_t xlo = make_smem_desc(xa + L.x_part + k * (L.x_part / 2));
 #pragma unroll
-              for (int e = 0; e < 4; ++e) tc_mma_f16(dtm, whi + 2 * e, xlo + 2 * e, p.idesc, 1u);
+              for (int e = 0; e < 4; ++e) tc_mma_f16_ts(dtm, whi + 8 * e, xlo + 2 * e, p.idesc, 1u);
             }
           }
           tc_commit(wfree + ws.slot);
           tc_commit(xfree + xs.slot);
           xs.next(p.nx);
-          ws.next(p.nw);
+          ws.next(kWBufs);
         }
         tc_commit(accfull + set);
       }

@@ -15,11 +15,9 @@
 //    one multiplication and two masks make the registers of two 8-column tiles (bytes 0 or 8 and 0 or 128).  The ranks
 //    come out in reverse, so the bytes of the Y word are reversed too (any common order of the contraction serves).
 //  * Row and column sums are products with an operand of ones.
-// Column order: the tile nt = 2 qh + x holds, at column n, q = 16 qh + 4 (n >> 1) + 2 x' + (n & 1) with x' = x, or
-// x ^ (n >> 2) where SWAP is set; a lane thus owns q = 16 qh + 4 t + {0..3} of every row, in two pairs (x = 0, 1).
-// Without SWAP the pairs are in order (8- or 16-byte global stores that fill 32-byte sectors); with SWAP the lanes t < 2
-// and t >= 2 write different halves of their four entries at a time, so that 4-byte stores into rows of 128
-// swizzled bytes touch every bank once.
+// Column order: the tile nt = 2 qh + x holds, at column n, q = 16 qh + 4 (n >> 1) + 2 x + (n & 1); a lane thus owns
+// q = 16 qh + 4 t + {0..3} of every row, in two pairs (x = 0, 1): 8- or 16-byte global stores that fill 32-byte sectors, or
+// the registers of a 16x256b tensor-memory store.
 #pragma once
 #include "bqq_common.cuh"
 
@@ -50,10 +48,9 @@ struct RebuildLane {
   uint32_t zsel[2];            // byte of tile x, zeros above it
   int zfrom;                   // plane lane of rank half 0 (rank half 1: + 16)
 };
-template <bool SWAP>
 __device__ __forceinline__ RebuildLane rebuild_lane(int lane) {
   const int g = lane >> 2, t = lane & 3;
-  const uint32_t e = (SWAP ? 2 * (g >> 2) : 0) + (g & 1);
+  const uint32_t e = g & 1;
   RebuildLane L;
   L.zsel[0] = 0x4440u | e;
   L.zsel[1] = 0x4440u | (e ^ 2u);

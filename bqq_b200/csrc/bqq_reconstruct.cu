@@ -222,7 +222,7 @@ bqq_reconstruct_kernel(const ReconParams p) {
     pdl_enter(p.pdl);
     const int grp = warp / kGroup, sub = warp % kGroup;
     const int g8 = lane >> 2, t4 = lane & 3;
-    const RebuildLane L = rebuild_lane<false>(lane);
+    const RebuildLane L = rebuild_lane(lane);
     const long long ldw = (long long)g.cw * g.Q;
     const long long here = (long long)sub * g.Q + g8 * ldw + 4 * t4;   // the lane's first entry inside a block
     RebuildAcc r;
