@@ -261,7 +261,7 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
         __syncwarp();
         tc_fence_after();
         if (there) {
-          rebuild_end(r, d * f);
+          rebuild_end(r, d * f, lane);
           // entry pairs of rows g + 8 rr: 32-bit columns 8 qh + 2 t + x of the lane's quarter, which is their order in K
           auto rows16 = [&](auto MT) {
             constexpr int mt = decltype(MT)::value;

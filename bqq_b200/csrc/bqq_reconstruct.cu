@@ -252,7 +252,7 @@ bqq_reconstruct_kernel(const ReconParams p) {
       if (!live) continue;
 
       // 32 x 32 entries: a lane holds four neighbouring columns of rows g8 + 8 rr in either half
-      rebuild_end(r, d);
+      rebuild_end(r, d, lane);
       WT* wp = reinterpret_cast<WT*>(p.W) + at;
       WT* lp = LO ? reinterpret_cast<WT*>(p.W_lo) + at : nullptr;
       const bool quad0 = p.quads && 4 * t4 + 4 <= cols, quad1 = p.quads && 4 * t4 + 20 <= cols;
