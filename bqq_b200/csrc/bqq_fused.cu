@@ -11,50 +11,67 @@ namespace bqq {
 // x in the kernel's column order, zeros in the padding; also clears the counters of the tiles for callers whose scratch is not
 // kept clean.  Eight columns per thread.  NP (formats of bqq_fused_kernel.cuh) = 1: fp16, bf16 rows scaled by a power of
 // two (the row's maximum maps to at most 2^14; unscale[m] = 1 / scale); 2: bf16; 3: bf16 hi and lo = the rest.
-template <int NP>
-__global__ void __launch_bounds__(256)
+// Bound: two round trips to x, the row's maximum first, and what the SM does meanwhile.  A CTA of 128 threads and 32 registers
+// (at most one per SM) shares the SM with a CTA of the fused kernel, which then rebuilds up to four stages of W beside it; one of
+// 256 threads and 46 registers kept that CTA out until it was done (4096 x 4096, 2 bit layers, 64 rows: 24.8 -> 21.3 us in
+// all; P = 96, Q = 40, r = 33, 5 rows 17.8 -> 14.3).  Rows of more than kPrepLong columns are more round trips
+// than a rebuild of four stages hides: CTAs of 256 threads, in front of the fused kernel (28672 columns, 32 rows: 282
+// against 293 us).
+constexpr int kPrepThreads = 128, kPrepWide = 256, kPrepLong = 16384;
+template <int NP, int T>
+__global__ void __launch_bounds__(T, T == kPrepThreads ? 16 : 1)
 fused_prep_kernel(const XSource xs, int M, Geom g, int Kp, uint16_t* __restrict__ hi, uint16_t* __restrict__ lo,
                   float* __restrict__ unscale, unsigned* __restrict__ zero, int nzero, unsigned* __restrict__ status) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (blockIdx.x == 0 && blockIdx.y == 0) {
-    for (int e = threadIdx.x; e < nzero; e += 256) zero[e] = 0u;
+    for (int e = threadIdx.x; e < nzero; e += T) zero[e] = 0u;
     if (status && threadIdx.x == 0) *status = 0u;
   }
   if (!hi) return;
+  constexpr int kWarps = T / 32;
+  __shared__ float part[kWarps];
   const int m = blockIdx.y;
-  __shared__ float part[8];
   float inv_rms = 1.f, scale = 1.f;
   if (NP != 1 && xs.mode == BQQ_PRO_RMSNORM) {
-    const float w = row_sumsq_share(xs, m, threadIdx.x, 256);
+    const float w = row_sumsq_share(xs, m, threadIdx.x, T);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = w;
     __syncthreads();
     float tot = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) tot += part[k];
+    for (int k = 0; k < kWarps; ++k) tot += part[k];
     inv_rms = rsqrtf(tot / (float)xs.n_in + xs.eps);
   }
   if (NP == 1 && unscale) {
     float top = 0.f;
-    if ((xs.n_in & 3) == 0) {
-      for (int n = 4 * threadIdx.x; n < xs.n_in; n += 1024) {
-        float v[4];
-        load_quad(xs.x, (size_t)m * xs.ld + n, xs.dtype, v);
-        top = fmaxf(top, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+    if ((xs.n_in & 3) == 0 && raw4_aligned(xs.x, (size_t)m * xs.ld, xs.dtype)) {
+      const uint16_t* row = reinterpret_cast<const uint16_t*>(xs.x) + (size_t)m * xs.ld;
+      constexpr int kAhead = 8;                       // in flight: one round trip for 4096 columns
+      for (int n0 = 4 * threadIdx.x; n0 < xs.n_in; n0 += 4 * T * kAhead) {
+        uint2 r[kAhead];                              // 16-bit types only
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+          r[k] = n0 + 4 * T * k < xs.n_in ? *reinterpret_cast<const uint2*>(row + n0 + 4 * T * k) : make_uint2(0u, 0u);
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+          float v[4];
+          raw4_to_float(make_uint4(r[k].x, r[k].y, 0u, 0u), xs.dtype, v);
+          top = fmaxf(top, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+        }
       }
     } else {
-      for (int n = threadIdx.x; n < xs.n_in; n += 256) top = fmaxf(top, fabsf(load_as_float(xs.x, (size_t)m * xs.ld + n, xs.dtype)));
+      for (int n = threadIdx.x; n < xs.n_in; n += T) top = fmaxf(top, fabsf(load_as_float(xs.x, (size_t)m * xs.ld + n, xs.dtype)));
     }
 #pragma unroll
     for (int e = 16; e > 0; e >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, e));
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = top;
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 8; ++k) top = fmaxf(top, part[k]);
+    for (int k = 0; k < kWarps; ++k) top = fmaxf(top, part[k]);
     scale = scale_from_bound(top);
     if (threadIdx.x == 0 && blockIdx.x == 0) unscale[m] = 1.f / scale;
   }
-  for (int k0 = (blockIdx.x * 256 + threadIdx.x) * 8; k0 < Kp; k0 += gridDim.x * 2048) {
+  for (int k0 = (blockIdx.x * T + threadIdx.x) * 8; k0 < Kp; k0 += gridDim.x * (8 * T)) {
     const int blk = k0 >> 5, c0 = k0 & 31;
     const int sub = blk & 3, s = blk >> 2;
     const int jg = s / g.QT, qt = s - jg * g.QT;
@@ -100,7 +117,7 @@ struct FusedPlan {
   size_t smem, partial_bytes, x_bytes;
 };
 
-constexpr size_t kMaxSmem = 227 * 1024;
+constexpr size_t kMaxSmem = 225 * 1024;            // leaves room for a CTA of the preparation
 inline size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
 FusedPlan make_plan(const Geom& g, int M, int NP, bool any_rows) {
@@ -228,8 +245,11 @@ int fused_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t l
                         prologue ? fusion->prologue : BQQ_PRO_NONE, g.in_features(), fusion ? fusion->eps : 0.f};
     cudaLaunchAttribute attr[1] = {pdl_attribute()};
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = direct ? dim3(1) : dim3((unsigned)std::min((pl.Kp + 2047) / 2048, 64), (unsigned)M);
-    cfg.blockDim = dim3(256);
+    const bool wide = !direct && xs.n_in > kPrepLong;
+    const int threads = wide ? kPrepWide : kPrepThreads, per = 8 * threads;
+    const int parts = std::min((pl.Kp + per - 1) / per, wide ? 64 : 148 / M);
+    cfg.gridDim = direct ? dim3(1) : dim3((unsigned)parts, (unsigned)M);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -237,7 +257,13 @@ int fused_launch(const BqqLayer* L, const void* x, int x_dtype, int M, int64_t l
     uint16_t* h = direct ? nullptr : xhi;
     unsigned* stw = clear ? status : nullptr;
     float* un = const_cast<float*>(p.row_unscale);
-    auto kern = NP == 1 ? fused_prep_kernel<1> : NP == 2 ? fused_prep_kernel<2> : fused_prep_kernel<3>;
+    auto kern = wide ? (NP == 1 ? fused_prep_kernel<1, kPrepWide> : NP == 2 ? fused_prep_kernel<2, kPrepWide> : fused_prep_kernel<3, kPrepWide>)
+                     : (NP == 1 ? fused_prep_kernel<1, kPrepThreads> : NP == 2 ? fused_prep_kernel<2, kPrepThreads> : fused_prep_kernel<3, kPrepThreads>);
+    // an SM keeps its split of L1 and shared memory until it is empty: the one that the fused kernel needs
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) {
+      cudaGetLastError();
+      return BQQ_ERR_CUDA;
+    }
     if (cudaLaunchKernelEx(&cfg, kern, xs, M, g, pl.Kp, h, xlo, un, counters, nzero, stw) != cudaSuccess) {
       cudaGetLastError();
       return BQQ_ERR_CUDA;

@@ -46,3 +46,18 @@ def test_fused_many_items(rw, cw, M):
     if M <= 16:
         parts = [_run(shard_rows(bq, k, 2).cuda(), X) for k in range(2)]
         assert torch.equal(torch.cat(parts, -1), y)
+
+
+@pytest.mark.parametrize('cw,Q,M', [(530, 32, 20), (530, 31, 3), (131, 128, 17), (40, 31, 74), (2, 36, 128)])
+def test_fused_rows_of_every_length(cw, Q, M):
+    """x staged by either preparation (rows of up to 16384 columns and longer ones), quads aligned or not."""
+    from bqq_b200.bqq_modules import BinaryQuadratic
+    Y, Z, A, _, X = synth_layer(1, 2, cw, 96, Q, 33, M, seed=cw + M)
+    bq = BinaryQuadratic(Y.float(), Z.float(), A).cuda()
+    for dt, tol in ((torch.float32, 1e-4), (torch.bfloat16, 1e-3 + 2 ** -8), (torch.float16, 1e-3 + 2 ** -10)):
+        Xd = X.to(dt)
+        ref = oracle_forward_t(Y, Z, A, None, Xd)
+        assert O.max_rel_err(_run(bq, Xd).float().cpu().numpy(), ref) < tol
+        wide = torch.zeros(M, cw * Q + 3, dtype=dt, device='cuda')
+        wide[:, 1:1 + cw * Q] = Xd.cuda()
+        assert O.max_rel_err(_run(bq, wide[:, 1:1 + cw * Q]).float().cpu().numpy(), ref) < tol
