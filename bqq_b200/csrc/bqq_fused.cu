@@ -120,6 +120,51 @@ struct FusedPlan {
 constexpr size_t kMaxSmem = 225 * 1024;            // leaves room for a CTA of the preparation
 inline size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
+// Estimated time (ns) of `tiles` tiles in chunks of `cs` stages, fitted to 27 layers and batches (8 to 224 tiles, 8 to 112
+// stages, 16 to 128 rows) in up to nine chunk lengths each: rounds of items over 148 SMs, an item no shorter than what moves its
+// sums, then the sum over the chunks of a tile by one CTA.
+long long chunk_cost(const Geom& g, int stages, int tiles, int N, int cs) {
+  const int chunks = (stages + cs - 1) / cs;
+  const long long rounds = ((long long)tiles * chunks + 147) / 148;
+  const long long item = cs * (870LL + g.bw * (g.RT == 1 ? 385 : 640)) + 1280 + 23 * N;
+  if (chunks == 1) return rounds * item;
+  return rounds * std::max(item, 3080LL + 25 * N) + 400 + (12LL * N * ((tiles + 147) / 148) + 30) * chunks;
+}
+
+// Chunk length of a layer, at most 32 chunks.  tiles = 0: the sum must not depend on the number of rows of W (a row shard
+// reproduces the whole layer bit for bit), so it is the length that is good for 16 to 112 tiles (2048 to 14336 rows) alike.
+// (us, length for 32 tiles -> this one, 16 rows: 2048 x 6144 b2 22.8 -> 15.6, 6144 x 2048 b3 19.1 -> 17.6, 14336 x 4096 b2
+// 60.8 -> 56.5.)  A thread keeps the lengths it used last: the search takes about as long as a launch.
+int chunk_length(const Geom& g, int stages, int tiles, int N) {
+  constexpr int kSeen = 32;
+  struct Seen { int stages, bw, RT, tiles, N, cs; };
+  static thread_local Seen seen[kSeen] = {};
+  Seen& m = seen[(unsigned)(stages * 31 + g.bw * 7 + g.RT + tiles * 13 + N) % kSeen];
+  if (m.cs && m.stages == stages && m.bw == g.bw && m.RT == g.RT && m.tiles == tiles && m.N == N) return m.cs;
+  static const int kTypical[4] = {16, 32, 48, 112};
+  const int* const set = tiles ? &tiles : kTypical;
+  const int n = tiles ? 1 : 4;
+  double least[4];
+  for (int k = 0; k < n; ++k) {
+    long long lo = -1;
+    for (int c = 1; c <= std::min(stages, 32); ++c) {
+      const long long v = chunk_cost(g, stages, set[k], N, (stages + c - 1) / c);
+      if (lo < 0 || v < lo) lo = v;
+    }
+    least[k] = (double)lo;
+  }
+  double best = -1.;
+  int cs = stages;
+  for (int c = std::min(stages, 32); c >= 1; --c) {
+    const int len = (stages + c - 1) / c;
+    double sum = 0.;
+    for (int k = 0; k < n; ++k) sum += (double)chunk_cost(g, stages, set[k], N, len) / least[k];
+    if (best < 0. || sum < best) { best = sum; cs = len; }
+  }
+  m = {stages, g.bw, g.RT, tiles, N, cs};
+  return cs;
+}
+
 FusedPlan make_plan(const Geom& g, int M, int NP, bool any_rows) {
   FusedPlan pl = {};
   pl.N = (M + 15) / 16 * 16;
@@ -144,19 +189,8 @@ FusedPlan make_plan(const Geom& g, int M, int NP, bool any_rows) {
   pl.stages = g.JG * g.QT;
   pl.Kp = pl.stages * kFusedStageCols;
   pl.tiles = (g.rw * g.PT + 3) / 4;
-  // Chunk length: the cheapest by estimated clocks - rounds of items over 148 SMs, each a fixed part and its stages, then
-  // the sum over the chunks by one CTA.  Up to 16 rows the sum must not depend on the number of rows of W (a row shard
-  // reproduces the whole layer bit for bit), so the estimate is made for 4096 rows there.
-  const long long tiles = any_rows ? 32 : pl.tiles;
-  long long best = -1;
-  for (int cs = 1; cs <= pl.stages; ++cs) {
-    const int chunks = (pl.stages + cs - 1) / cs;
-    if (chunks > 32) continue;
-    const long long rounds = (tiles * chunks + 147) / 148;
-    const long long item = 1000 + (chunks > 1 ? 25LL * pl.N : 8LL * pl.N) + (long long)cs * (g.bw * RT * 1200LL + 600);
-    const long long cost = rounds * item + (chunks > 1 ? 2500 + 16LL * chunks * M * ((tiles + 147) / 148) : 0);
-    if (best < 0 || cost < best) { best = cost; pl.chunk_stages = cs; pl.chunks = chunks; }
-  }
+  pl.chunk_stages = chunk_length(g, pl.stages, any_rows ? 0 : pl.tiles, pl.N);
+  pl.chunks = (pl.stages + pl.chunk_stages - 1) / pl.chunk_stages;
   pl.partial_bytes = pl.chunks > 1 ? up256((size_t)pl.tiles * pl.chunks * pl.N * kFusedTile * 4) : 0;
   pl.x_bytes = up256((size_t)M * pl.Kp * 2) + 1024;         // and the factors of the rows
   pl.ok = true;
