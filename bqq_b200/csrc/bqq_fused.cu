@@ -168,7 +168,10 @@ int chunk_length(const Geom& g, int stages, int tiles, int N) {
 FusedPlan make_plan(const Geom& g, int M, int NP, bool any_rows) {
   FusedPlan pl = {};
   pl.N = (M + 15) / 16 * 16;
-  if (pl.N > (NP == 3 ? 64 : kFusedMaxN)) return pl;
+  if (pl.N > kFusedMaxN) return pl;
+  // three products over columns that are a third or more padding cost more than a GEMM over those that exist (1600 x 6000,
+  // Q = 40, fp32: 62 against 55 us at 128 rows, even at 96)
+  if (NP == 3 && pl.N > 96 && 64 * g.QT > 3 * g.Q) return pl;
   const int RT = g.RT;
   // Shared memory: at least two of everything, with as many bit layers per plane stage as that leaves room for; then deeper
   // rings while there is room, x first (a round trip for x is longer than a stage).

@@ -14,7 +14,7 @@
 // helpers: plane words by TMA ([Y of all row blocks | Z of all] [bit] in a stage), coefficients as floats, x by TMA,
 // tcgen05 issue.  W is operand A and lives in tensor memory (lane = row, two neighbouring k per column): the registers of a
 // finished 32x32 block are what two 16x256b stores take, against sixteen 4-byte stores into swizzled shared memory, a
-// proxy fence and up to 128 KB of buffers before.  Three or four W buffers, two sets of accumulators D[128 rows of W][N
+// proxy fence and up to 128 KB of buffers before.  Two to four W buffers, two sets of accumulators D[128 rows of W][N
 // rows of x] beside them.
 // Formats, accumulated in fp32 (NP products per tile):
 //   1  W in fp16, x in fp16: 16-bit x of more than 16 rows.  Every block of 32 rows of an item is scaled by a power of two
@@ -182,14 +182,14 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
   const uint32_t acc_cols = (uint32_t)(p.N <= 16 ? 16 : p.N <= 32 ? 32 : p.N <= 64 ? 64 : 128);
   constexpr uint32_t kWPart = kFusedStageCols / 2;                      // tensor-memory columns of a W buffer: hi, then lo
   constexpr uint32_t kWCols = NP == 1 ? kWPart : 2 * kWPart;
-  constexpr int kWBufs = NP == 1 ? 4 : 3;
+  const int wbufs = NP == 1 ? 4 : acc_cols > 64 ? 2 : 3;
   constexpr uint32_t tmem_cols = 512;
-  static_assert((NP == 1 ? 256 : NP == 2 ? 128 : 128) + kWBufs * kWCols <= tmem_cols, "");
+  static_assert(256 + 4 * kWPart <= tmem_cols && 256 + 2 * 2 * kWPart <= tmem_cols && 128 + 3 * 2 * kWPart <= tmem_cols, "");
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.ns; ++s) { mbar_init(full + s, 1 + 32); mbar_init(used + s, kFusedWarps); }
     for (int s = 0; s < p.nx; ++s) { mbar_init(xfull + s, 1); mbar_init(xfree + s, 1); }
-    for (int s = 0; s < kWBufs; ++s) { mbar_init(wfull + s, kFusedWarps); mbar_init(wfree + s, 1); }
+    for (int s = 0; s < wbufs; ++s) { mbar_init(wfull + s, kFusedWarps); mbar_init(wfree + s, 1); }
     for (int s = 0; s < 2; ++s) {
       mbar_init(scaled + s, 4);
       mbar_init(accfull + s, 1);
@@ -257,7 +257,7 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
           if (lane == 0) mbar_arrive(used + ps.slot);
           ps.next(p.ns);
         }
-        if (wn >= kWBufs) wait(wfree + ws.slot, ws.phase ^ 1u);
+        if (wn >= wbufs) wait(wfree + ws.slot, ws.phase ^ 1u);
         __syncwarp();
         tc_fence_after();
         if (there) {
@@ -297,7 +297,7 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(wfull + ws.slot);
-        ws.next(kWBufs);
+        ws.next(wbufs);
         ++wn;
       }
     }
@@ -561,7 +561,7 @@ bqq_fused_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_consta
           tc_commit(wfree + ws.slot);
           tc_commit(xfree + xs.slot);
           xs.next(p.nx);
-          ws.next(kWBufs);
+          ws.next(wbufs);
         }
         tc_commit(accfull + set);
       }
