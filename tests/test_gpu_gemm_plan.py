@@ -38,3 +38,21 @@ def test_pairs_and_panels(rw, cw, M, dtype):
     tol = 1e-4 if dtype == torch.float32 else 1e-3 + (2 ** -8 if dtype == torch.bfloat16 else 2 ** -10)
     assert ((y - ref).abs().max() / ref.abs().max()).item() < tol
     check_status()
+
+
+@pytest.mark.parametrize('cw', [4, 33, 65])
+@pytest.mark.parametrize('M', [130, 700])
+def test_rows_staged_from_any_place(cw, M):
+    """x whose rows are not aligned to four elements, or not a multiple of a block's columns, takes the staging kernel."""
+    from bqq_b200.bqq_modules import BinaryQuadratic
+    Y, Z, A, _, X = synth_layer(2, 3, cw, 32, 32, 32, M, seed=cw + M)
+    bq = BinaryQuadratic(Y.float(), Z.float(), A).cuda()
+    for dt, tol in ((torch.float32, 1e-4), (torch.bfloat16, 1e-3 + 2 ** -8), (torch.float16, 1e-3 + 2 ** -10)):
+        Xd = X.to(dt)
+        ref = oracle_forward_t(Y, Z, A, None, Xd)
+        for skip, pitch in ((0, 0), (1, 3), (8, 8), (4, 5)):
+            wide = torch.zeros(M, cw * 32 + 16 + pitch, dtype=dt, device='cuda')
+            wide[:, skip:skip + cw * 32] = Xd.cuda()
+            with torch.no_grad():
+                y = bq(wide[:, skip:skip + cw * 32])
+            assert O.max_rel_err(y.float().cpu().numpy(), ref) < tol
