@@ -66,7 +66,9 @@ size_t decode_counter_bytes() { return kCounterBytes; }
 
 // The fused rebuild-and-multiply route costs the same for 2 and for 16 rows, the decode kernel about 9 us + 23 us per four
 // rows (4096 x 14336, 3 bit layers: 34 / 56 / 79 / 101 us against 62 us).  It is taken where it is the faster one: with 9
-// rows or more of patches of one block (2048 x 2048, 2 bit layers: 13.5 against 9.4 us; 14336 x 4096 is even), with 13 or
+// rows or more of patches of one block (2048 x 2048, 2 bit layers: 13.5 against 8.6 us; 14336 x 4096 is even), with 5 or
+// more (two passes of the decode kernel) where there are few columns at every height (28672 x 1024, 2 bit layers: 36 against
+// 33 us, 2048 x 1024: 9.2 against 6.2) or four bit layers share a block's end (14336 x 2048: 46 against 43; 14336 x 4096: 70 against 72), with 13 or
 // more of 2 x 2 blocks of two rank blocks (8192 x 28672, 3 bit layers 315 against 300 us, 4096 x 4096 32 against 24; with one
 // rank block the decode kernel shares its operands better), and wherever the patch geometry runs in a decode variant with half
 // as many blocks again as it has (P = 96, Q = 40, r = 33: 24 against 14 us at 5 rows).  The rule knows nothing of the
@@ -75,7 +77,8 @@ static bool fused_decode(const Geom& g, int M) {
   int v = 0;
   while (v < 3 && !(g.PT <= kVariantPT[v] && g.QT <= kVariantQT[v] && g.RT <= kVariantRT[v])) ++v;
   const int padded = kVariantRT[v] * (kVariantPT[v] + kVariantQT[v]), own = g.RT * (g.PT + g.QT);
-  const bool faster = g.PT * g.QT * g.RT == 1 ? M >= 9 : (M >= 2 && 2 * padded >= 3 * own) || (M >= 13 && g.PT == 2 && g.QT == 2 && g.RT == 2);
+  const bool faster = g.PT * g.QT * g.RT == 1 ? M >= 9 || (M >= 5 && (g.JG <= 8 || (g.bw >= 4 && g.JG <= 16)))
+                                               : (M >= 2 && 2 * padded >= 3 * own) || (M >= 13 && g.PT == 2 && g.QT == 2 && g.RT == 2);
   return faster && fused_counter_words(g) < (size_t)kMaxCounters && fused_workspace_bytes(g, M) > 0;
 }
 

@@ -159,7 +159,7 @@ int bqq_repack_u8_planes(const uint8_t* Y_packed, const uint8_t* Z_packed, const
  *   required.  Calls sharing a workspace
  *   must not overlap on the GPU.  Results do not depend on the number of row
  *   patches: a row shard reproduces its slice of the full output bit for bit.
- *   From 9 rows on (13 or, where the kernel would pad the patch geometry badly, 2)
+ *   From 9 rows on (2 to 13 depending on the patch geometry, bit layers and columns)
  *   W is instead rebuilt tile by tile in tensor memory and multiplied by tcgen05 at
  *   once, W as a pair of bf16 and x as it is or as a pair.
  * bqq_forward_prefill: any M; up to 128 rows the same with W and x in fp16 (a pair
@@ -233,7 +233,7 @@ int bqq_prefill_status(const void* workspace, void* stream);
  * Number of kernels one bqq_forward_decode call enqueues for this layer shape and
  * M (1 or 2: short single-chunk layers at M = 1 prepare x inside the decode
  * kernel, and aligned bf16 rows of 32-column patches are multiplied as they are
- * from 9 rows on; all others launch a preparation kernel first); negative BQQ_ERR_* for
+ * on the route for more rows; all others launch a preparation kernel first); negative BQQ_ERR_* for
  * bad arguments.  For launch accounting; the reference has no such query.
  */
 int bqq_decode_launches(const BqqDims* dims, int M);

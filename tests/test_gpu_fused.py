@@ -17,7 +17,7 @@ def _run(bq, X):
 
 @pytest.mark.parametrize('shape', [(2, 3, 5, 32, 32, 32), (9, 5, 7, 32, 32, 32), (1, 3, 5, 96, 40, 33), (3, 4, 6, 64, 64, 64),
                                    (2, 7, 3, 40, 128, 16), (2, 9, 40, 32, 32, 32)])
-@pytest.mark.parametrize('M', [8, 9, 12, 13, 16, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize('M', [4, 5, 8, 9, 12, 13, 16, 17, 33, 64, 65, 128])
 def test_fused_against_oracle(shape, M):
     from bqq_b200.bqq_modules import BinaryQuadratic, check_status
     Y, Z, A, bias, X = synth_layer(*shape, M, seed=sum(shape) + M, bias=True)
